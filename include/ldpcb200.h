@@ -283,18 +283,22 @@ int ldpc_set_circulant(ldpc_handle* h, const ldpc_circ_config* c);
  * type is float (fp64 = 0; alpha = 1, beta = 0 then reproduces the plain fp32 decoder bit for bit)
  * or double (fp64 = 1, for checking the adjoint against finite differences; rate 1/2 and 4/5 at
  * K = 1024 only): every array argument below is of that type.  All pointers are device memory owned
- * by the caller; the workspace holds the activation checkpoints between the forward and the
+ * by the caller; the workspace holds the activations between the forward and the
  * backward call of the same frames.  Work is queued on the stream; the calls do not wait for it. */
 typedef struct {
     int32_t n_iter;              /* T, 1..64 */
     int32_t n_classes;           /* C, 1..64 */
-    int32_t ckpt_every;          /* iterations between activation checkpoints, 1..T */
+    int32_t ckpt_every;          /* 1..T: sizes the workspace (ldpc_wdec_workspace_bytes) */
     int32_t post_all;            /* 1: posteriors after every iteration [T][n][N]; 0: after the last [1][n][N] */
     int32_t fp64;                /* 0: float arrays; 1: double arrays */
     int32_t reserved0;
     int32_t edge_class[12][18];  /* class of edge e of layer l */
 } ldpc_wdec_config;
 
+/* Workspace for n_frames: at most what checkpoints of L and the messages every ckpt_every iterations, the
+ * rows of ckpt_every iterations and two message arrays take.  Within it the forward call keeps the rows
+ * (q of every edge) of as many of the last iterations as fit; the backward call runs only the iterations
+ * before those again. */
 int64_t ldpc_wdec_workspace_bytes(const ldpc_handle* h, const ldpc_wdec_config* c, int64_t n_frames);
 
 /* d_llr [n][N-P] channel LLRs, d_alpha/d_beta [T][C] -> d_post (see post_all). */

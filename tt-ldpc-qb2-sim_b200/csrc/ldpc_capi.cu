@@ -1322,11 +1322,25 @@ extern "C" int ldpc_batch_run(ldpc_batch* b, const ldpc_run_params* params, cons
 }
 
 // ----------------------------------------------------------------------------- weighted decoder (training)
-struct WLayout {
-    size_t ckpt, rwork, stash, gr, total;  // offsets (elements of the real type) and total bytes
-};
+static void wparams_fill(const ldpc_handle* h, const ldpc_wdec_config* c, int64_t n, WParams* p) {
+    memset(p, 0, sizeof *p);
+    for (int l = 0; l < QC_LAYERS; ++l)
+        for (int e = 0; e < QC_DMAX; ++e) p->edge[l][e] = h->blk_off[l][e] + h->shift[l][e];
+    memcpy(p->edge_class, c->edge_class, sizeof p->edge_class);
+    p->n_vars = h->N;
+    p->n_tx = h->N - h->P;
+    p->n_iter = c->n_iter;
+    p->n_classes = c->n_classes;
+    p->post_all = c->post_all ? 1 : 0;
+    p->n_frames = (int32_t)n;
+    p->row_uniform = 1;
+    for (int l = 0; l < QC_LAYERS; ++l)
+        for (int e = 1; e < (l < 4 ? QC_DEG_LOW : h->D); ++e)
+            if (c->edge_class[l][e] != c->edge_class[l][0]) p->row_uniform = 0;
+}
 
-static int wcheck(const ldpc_handle* h, const ldpc_wdec_config* c, int64_t n, WLayout* lay) {
+// Checks a configuration; fills the kernel parameters and the workspace's layout and size (bytes).
+static int wcheck(const ldpc_handle* h, const ldpc_wdec_config* c, int64_t n, WParams* p, size_t* bytes) {
     if (!h || !c) return fail(LDPC_EINVAL, "handle or config is NULL");
     if (h->kind != LDPC_KERNEL_QC) return fail(LDPC_ENOTSUP, "the weighted decoder needs a QC code");
     const int rb = c->fp64 ? 8 : 4;
@@ -1340,60 +1354,42 @@ static int wcheck(const ldpc_handle* h, const ldpc_wdec_config* c, int64_t n, WL
         for (int e = 0; e < (l < 4 ? QC_DEG_LOW : h->D); ++e)
             if (c->edge_class[l][e] < 0 || c->edge_class[l][e] >= c->n_classes)
                 return fail(LDPC_EINVAL, "edge class of layer %d edge %d out of range", l, e);
-    const size_t E = (size_t)h->Z * (4 * QC_DEG_LOW + 8 * h->D);
-    const size_t n_ckpt = (c->n_iter + c->ckpt_every - 1) / c->ckpt_every;
-    lay->ckpt = 0;
-    lay->rwork = lay->ckpt + n_ckpt * n * (h->N + E);
-    lay->stash = lay->rwork + n * E;
-    lay->gr = lay->stash + (size_t)n * c->ckpt_every * E;
-    lay->total = (lay->gr + n * E) * rb;
+    wparams_fill(h, c, n, p);
+    *bytes = weighted_plan(p, h->Z, h->D, c->ckpt_every, h->n_sm, rb);
     return 0;
 }
 
-static void wparams_fill(const ldpc_handle* h, const ldpc_wdec_config* c, int64_t n, WParams* p) {
-    memset(p, 0, sizeof *p);
-    memcpy(p->blk_off, h->blk_off, sizeof p->blk_off);
-    memcpy(p->shift, h->shift, sizeof p->shift);
-    memcpy(p->edge_class, c->edge_class, sizeof p->edge_class);
-    int32_t off = 0;
-    for (int l = 0; l < QC_LAYERS; ++l) {
-        p->layer_off[l] = off;
-        off += h->Z * (l < 4 ? QC_DEG_LOW : h->D);
-    }
-    p->n_vars = h->N;
-    p->n_tx = h->N - h->P;
-    p->n_edges = off;
-    p->n_iter = c->n_iter;
-    p->n_classes = c->n_classes;
-    p->ckpt_every = c->ckpt_every;
-    p->post_all = c->post_all ? 1 : 0;
-    p->n_frames = (int32_t)n;
+static void wworkspace(WParams* p, void* d_ws, size_t rb) {
+    char* ws = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(d_ws) + W_ALIGN - 1) / W_ALIGN * W_ALIGN);
+    p->stash = ws;
+    p->ckpt = ws + p->off_ckpt * rb;
+    p->gr = ws + p->off_gr * rb;
+    p->save = ws + p->off_save * rb;
+    p->used = reinterpret_cast<int32_t*>(ws + p->off_used * rb);
 }
 
 extern "C" int64_t ldpc_wdec_workspace_bytes(const ldpc_handle* h, const ldpc_wdec_config* c, int64_t n) {
-    WLayout lay;
-    int rc = wcheck(h, c, n, &lay);
-    return rc ? rc : (int64_t)lay.total;
+    WParams p;
+    size_t bytes = 0;
+    int rc = wcheck(h, c, n, &p, &bytes);
+    return rc ? rc : (int64_t)bytes;
 }
 
 extern "C" int ldpc_wdec_forward(ldpc_handle* h, const ldpc_wdec_config* c, const void* d_llr, int64_t n,
                                  const void* d_alpha, const void* d_beta, void* d_post, void* d_ws, void* stream) {
-    WLayout lay;
+    WParams p;
+    size_t bytes = 0;
     int rc;
-    if ((rc = wcheck(h, c, n, &lay))) return rc;
+    if ((rc = wcheck(h, c, n, &p, &bytes))) return rc;
     if (n && (!d_llr || !d_alpha || !d_beta || !d_post || !d_ws)) return fail(LDPC_EINVAL, "NULL device pointer");
     CU(cudaSetDevice(h->device));
-    WParams p;
-    wparams_fill(h, c, n, &p);
-    char* ws = static_cast<char*>(d_ws);
-    const size_t rb = c->fp64 ? 8 : 4;
+    const int rb = c->fp64 ? 8 : 4;
     p.llr = d_llr;
     p.alpha = d_alpha;
     p.beta = d_beta;
     p.post = d_post;
-    p.ckpt = ws + lay.ckpt * rb;
-    p.rwork = ws + lay.rwork * rb;
-    if ((rc = weighted_forward(p, h->Z, h->D, (int)rb, static_cast<cudaStream_t>(stream), g_err))) return rc;
+    wworkspace(&p, d_ws, rb);
+    if ((rc = weighted_launch(p, h->Z, h->D, rb, true, h->n_sm, static_cast<cudaStream_t>(stream), g_err))) return rc;
     h->launches += n ? 1 : 0;
     return 0;
 }
@@ -1401,9 +1397,10 @@ extern "C" int ldpc_wdec_forward(ldpc_handle* h, const ldpc_wdec_config* c, cons
 extern "C" int ldpc_wdec_backward(ldpc_handle* h, const ldpc_wdec_config* c, int64_t n, const void* d_alpha,
                                   const void* d_beta, const void* d_gpost, void* d_galpha, void* d_gbeta,
                                   void* d_gllr, void* d_ws, void* stream) {
-    WLayout lay;
+    WParams p;
+    size_t bytes = 0;
     int rc;
-    if ((rc = wcheck(h, c, n, &lay))) return rc;
+    if ((rc = wcheck(h, c, n, &p, &bytes))) return rc;
     if (!d_alpha || !d_beta || !d_galpha || !d_gbeta || (n && (!d_gpost || !d_ws)))
         return fail(LDPC_EINVAL, "NULL device pointer");
     CU(cudaSetDevice(h->device));
@@ -1412,20 +1409,14 @@ extern "C" int ldpc_wdec_backward(ldpc_handle* h, const ldpc_wdec_config* c, int
     const size_t tc = (size_t)c->n_iter * c->n_classes * rb;
     CU(cudaMemsetAsync(d_galpha, 0, tc, s));
     CU(cudaMemsetAsync(d_gbeta, 0, tc, s));
-    WParams p;
-    wparams_fill(h, c, n, &p);
-    char* ws = static_cast<char*>(d_ws);
     p.alpha = d_alpha;
     p.beta = d_beta;
-    p.ckpt = ws + lay.ckpt * rb;
-    p.rwork = ws + lay.rwork * rb;
-    p.stash = ws + lay.stash * rb;
-    p.gr = ws + lay.gr * rb;
     p.gpost = d_gpost;
     p.galpha = d_galpha;
     p.gbeta = d_gbeta;
     p.gllr = d_gllr;
-    if ((rc = weighted_backward(p, h->Z, h->D, rb, s, g_err))) return rc;
+    wworkspace(&p, d_ws, rb);
+    if ((rc = weighted_launch(p, h->Z, h->D, rb, false, h->n_sm, s, g_err))) return rc;
     h->launches += n ? 1 : 0;
     return 0;
 }
