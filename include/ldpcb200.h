@@ -188,10 +188,11 @@ int ldpc_snr_bins(ldpc_handle* h, uint64_t* out);
  * degree-D layers in a loop that is not unrolled, its descriptors read by layer index (rate 4/5 at
  * K = 1024 and 4096, rate 2/3 at K = 1024: any matrix of that shape); layouts 3 and 4 are the
  * general kernels'.
- * All zero restores the default.
+ * All zero restores the default, which depends on the frames of the call, the storage mode and the
+ * options (every shape gives the same bits).
  * LDPC_ENOTSUP if the shape is not built for this code.  Used by the autotuner
- * (ldpcb200.capi.Decoder.autotune).  Options with no QC variant built (e.g. clips on a K = 16384
- * code) run on the general kernel. */
+ * (ldpcb200.capi.Decoder.autotune).  Options with no QC variant built (e.g. clips with fp32 storage)
+ * run on the general kernel. */
 int ldpc_set_launch_shape(ldpc_handle* h, int storage, int rows_per_thread, int frames_per_cta,
                           int min_ctas_per_sm, int global_messages);
 

@@ -49,6 +49,12 @@ void register_qc_table(QcTable* t) {
     g_tables = t;
 }
 const QcTable* qc_tables() { return g_tables; }
+static const QcDefaults* g_defaults = nullptr;
+void register_qc_defaults(QcDefaults* t) {
+    t->next = g_defaults;
+    g_defaults = t;
+}
+const QcDefaults* qc_defaults() { return g_defaults; }
 }  // namespace ldpcb200
 
 static const void* find_qc(const QcKey& k) {
@@ -343,10 +349,25 @@ static const void* find_shape(const ldpc_handle* h, int storage, int algo, int c
     return find_qc(QcKey{h->Z, h->D, R, F, storage, algo, clip, ext, B, G});
 }
 
-// The default shape of a numerics variant: one row per thread and one frame per CTA with messages in
-// registers when that is built, else the first shape built for it (e.g. the global-message kernel of
-// a K = 16384 code).
-static bool default_shape(const ldpc_handle* h, int storage, int algo, int clip, int ext, int s[4]) {
+static bool shape_in_scratch(int G) { return G == 1 || G == 5 || G == 7; }  // messages in global memory
+
+// The default shape of a numerics variant for a call of n frames: the first line of the defaults that
+// applies (QcDefault), else one row per thread and one frame per CTA with messages in registers when that is
+// built, else the first shape built for it (e.g. the global-message kernel of a K = 16384 code).
+// scratch = false leaves out the lines that need a message scratch.
+static bool default_shape(const ldpc_handle* h, int storage, int algo, int clip, int ext, uint32_t n, bool scratch,
+                          int s[4]) {
+    for (int own = 1; own >= 0; --own)
+        for (const QcDefaults* t = qc_defaults(); t; t = t->next)
+            for (int i = 0; i < t->count; ++i) {
+                const QcDefault& d = t->entries[i];
+                if (d.Z != h->Z || d.D != h->D || d.mode != storage || d.algo != (own ? algo : -1) || n < d.min_frames ||
+                    (!scratch && shape_in_scratch(d.G)) ||
+                    !find_shape(h, storage, algo, clip, ext, d.R, d.F, d.B, d.G))
+                    continue;
+                s[0] = d.R; s[1] = d.F; s[2] = d.B; s[3] = d.G;
+                return true;
+            }
     if (find_shape(h, storage, algo, clip, ext, 1, 1, 0, 0)) {
         s[0] = 1; s[1] = 1; s[2] = 0; s[3] = 0;
         return true;
@@ -365,7 +386,7 @@ static bool default_shape(const ldpc_handle* h, int storage, int algo, int clip,
 
 static bool default_shape_exists(const ldpc_handle* h, int storage, int algo) {
     int s[4];
-    return default_shape(h, storage, algo, 0, 0, s);
+    return default_shape(h, storage, algo, 0, 0, 0, true, s);
 }
 
 extern "C" int ldpc_set_weights(ldpc_handle* h, const float* alpha, const float* beta, int n_iter, int n_classes,
@@ -568,6 +589,10 @@ struct QcLaunch {
 
 static double code_rate(const ldpc_handle* h) { return (double)(h->N - h->M) / (double)(h->N - h->P); }
 
+static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void* fn, const int* sh, bool wrow, bool ext,
+                            uint32_t n, uint64_t first, const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf,
+                            int32_t* d_be, double grid_frac, QcLaunch* out);
+
 // Chooses the QC kernel for these numerics and shape and fills its launch; grid_frac < 1 gives the
 // launch that share of the GPU's resident CTA slots (for kernels that run side by side).
 static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32_t n, uint64_t first,
@@ -575,6 +600,7 @@ static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32
                       double grid_frac, QcLaunch* out) {
     const bool clip = p->l_max > 0.0f || p->r_max > 0.0f || p->l_post_max > 0.0f;
     int sh[4];
+    bool chosen = false, scratch = true;
     // the handle's shape for this storage, else the default shape of the algorithm
     auto lookup = [&](int algo) -> const void* {
         int s[4] = {h->shape[p->storage][0], h->shape[p->storage][1], h->shape[p->storage][2],
@@ -582,10 +608,11 @@ static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32
         const void* f = nullptr;
         if (s[0] || s[1] || s[2] || s[3])
             f = find_shape(h, p->storage, algo, clip, ext, s[0] ? s[0] : 1, s[1] ? s[1] : 1, s[2], s[3]);
+        chosen = f != nullptr;
         if (f) {
             s[0] = s[0] ? s[0] : 1;
             s[1] = s[1] ? s[1] : 1;
-        } else if (default_shape(h, p->storage, algo, clip, ext, s)) {
+        } else if (default_shape(h, p->storage, algo, clip, ext, n, scratch, s)) {
             f = find_shape(h, p->storage, algo, clip, ext, s[0], s[1], s[2], s[3]);
         }
         if (f) std::copy(s, s + 4, sh);
@@ -595,6 +622,20 @@ static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32
     const bool wrow = p->algo == LDPC_ALGO_WAMIN && h->w_row && lookup(ALGO_WROW);
     const void* fn = lookup(wrow ? ALGO_WROW : p->algo);
     if (!fn) return LDPC_ENOTSUP;  // the caller falls back to the general kernel
+    int rc = prepare_qc_shape(h, p, fn, sh, wrow, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, grid_frac, out);
+    if (rc == LDPC_ENOMEM && !chosen && shape_in_scratch(sh[3])) {
+        // no memory for a default shape's message scratch: the default without one, where there is one
+        scratch = false;
+        fn = lookup(wrow ? ALGO_WROW : p->algo);
+        if (fn && !shape_in_scratch(sh[3]))
+            rc = prepare_qc_shape(h, p, fn, sh, wrow, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, grid_frac, out);
+    }
+    return rc;
+}
+
+static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void* fn, const int* sh, bool wrow, bool ext,
+                            uint32_t n, uint64_t first, const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf,
+                            int32_t* d_be, double grid_frac, QcLaunch* out) {
     const int R = sh[0], F = sh[1], G = sh[3];
     QcParams& qp = out->qp;
     memset(&qp, 0, sizeof qp);
@@ -686,7 +727,7 @@ static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32
     out->block = T;
     out->smem = smem;
     if (grid == 0) return 0;
-    if (G == 1 || G == 5 || G == 7) {
+    if (shape_in_scratch(G)) {
         int rc;
         const size_t rsz = p->storage == LDPC_STORE_FP32 ? 4 : 2;
         if ((rc = ensure_cap(&h->d_rmsg, &h->rmsg_cap, grid * F * (size_t)qp.slot_elems * rsz))) return rc;

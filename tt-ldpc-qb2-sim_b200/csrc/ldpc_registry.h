@@ -32,6 +32,24 @@ struct QcTable {
     const QcTable* next;
 };
 
+// Launch shape used when the caller has set none: for a call of at least min_frames frames, shape (R, F, B,
+// G) of storage mode `mode`; algo -1 stands for every algorithm.  The lines for the algorithm itself come
+// before those for every algorithm, each in table order, and the first whose kernel is built for the
+// call's options (and offered for the matrix) is taken.  Every shape gives the same bits, so the lines lie
+// where the measured times cross.
+struct QcDefault {
+    int Z, D, mode, algo;
+    uint32_t min_frames;
+    int R, F, B, G;
+};
+struct QcDefaults {
+    const QcDefault* entries;
+    int count;
+    const QcDefaults* next;
+};
+void register_qc_defaults(QcDefaults* t);
+const QcDefaults* qc_defaults();
+
 // Linked at static-initialisation time by each instantiation unit.
 void register_qc_table(QcTable* t);
 const QcTable* qc_tables();
@@ -75,6 +93,27 @@ const QcTable* qc_tables();
      reinterpret_cast<const void*>(                                            \
          &::ldpcb200::qc_decode_kernel<Z, D, 1, 2, MODE, ::ldpcb200::ALGO_AMIN, false, EXT, B, true>)}
 
+// Layout 5 or 7 with the clips compiled in for a variant without clips: with infinite caps they leave every
+// value but NaN as it is, and a NaN posterior (from a NaN channel LLR) becomes -inf, as in the general kernel
+// these codes' caller-supplied LLRs ran on before.
+#define LDPC_QC_ENTRY_GF_NAN(Z, D, R, F, MODE, ALGO, EXT, B, FIX)             \
+    {{Z, D, R, F, MODE, ALGO, 0, EXT, B, 5},                                   \
+     reinterpret_cast<const void*>(                                            \
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, true, EXT, B, false, true, false, FIX>)}
+#define LDPC_QC_ENTRY_GR_NAN(Z, D, R, F, MODE, ALGO, EXT, B)                   \
+    {{Z, D, R, F, MODE, ALGO, 0, EXT, B, 7},                                   \
+     reinterpret_cast<const void*>(                                            \
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, true, EXT, B, false, true, false, -1, true>)}
+
+#define LDPC_QC_DEFAULTS(name)                                                           \
+    namespace {                                                                          \
+    struct name##_reg {                                                                  \
+        name##_reg() {                                                                   \
+            static ::ldpcb200::QcDefaults t{name, (int)(sizeof(name) / sizeof(name[0])), nullptr}; \
+            ::ldpcb200::register_qc_defaults(&t);                                        \
+        }                                                                                \
+    } name##_reg_instance;                                                               \
+    }
 #define LDPC_QC_REGISTER(name)                                                           \
     namespace {                                                                          \
     struct name##_reg {                                                                  \

@@ -18,5 +18,23 @@ static const QcEntry qc_circ[] = {
     // K = 16384 (Z = 2048): check messages in global memory, 512 threads x 4 rows
     LDPC_QC_ENTRY_G(2048, 6, 4, 1, STORE_BF16, ALGO_CIRC, false, false, 0),
     LDPC_QC_ENTRY_G(2048, 6, 4, 1, STORE_BF16, ALGO_CIRC, false, true, 0),
+    // layout 6: the code's layer descriptors compiled in
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_BF16, ALGO_CIRC, false, false, 5, 5),
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_BF16, ALGO_CIRC, false, true, 5, 5),
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP32, ALGO_CIRC, false, false, 5, 5),
+    LDPC_QC_ENTRY_RF(512, 6, 1, 1, STORE_BF16, ALGO_CIRC, false, false, 2, 6),
+    LDPC_QC_ENTRY_RF(512, 6, 1, 1, STORE_BF16, ALGO_CIRC, false, true, 2, 6),
 };
 LDPC_QC_REGISTER(qc_circ)
+
+// Defaults (us of the kernel at 440 / 100000 frames, 25000 for K = 4096, 2.04 dB): bf16 layout 6 54.4 / 6734,
+// offset table 55.6 / 6934, parameters 56.4 / 8023; fp32 44.6 / 5315 against 46.4 / 5917; K = 4096 148 / 6911
+// against 164 / 8017, but one frame 56.7 against 52.5.  K = 16384 keeps the parameter kernel: with the
+// descriptors compiled in it spills and takes 1.14 times as long.
+static const QcDefault qc_circ_default[] = {
+    {128, 6, STORE_BF16, ALGO_CIRC, 0, 1, 1, 5, 6},
+    {128, 6, STORE_BF16, ALGO_CIRC, 440, 1, 1, 0, 2},
+    {128, 6, STORE_FP32, ALGO_CIRC, 440, 1, 1, 5, 6},
+    {512, 6, STORE_BF16, ALGO_CIRC, 300, 1, 1, 2, 6},
+};
+LDPC_QC_DEFAULTS(qc_circ_default)

@@ -48,5 +48,26 @@ static const QcEntry qc_r45k1[] = {
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_AMIN, false, false, 24),
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_AMIN, false, false, 16),
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP16, ALGO_AMIN, false, false, 16),
+    // the storages' fastest shapes for caller-supplied LLRs
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_AMIN, false, true, 16),
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP16, ALGO_AMIN, false, true, 16),
+    LDPC_QC_ENTRY_GR_NAN(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, 24),
+    // the same for the -n and clip options
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_NMS, false, false, 16),
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 16),
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_NMS, false, true, 16),
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 16),
 };
 LDPC_QC_REGISTER(qc_r45k1)
+
+// Default shapes (us of the kernel at 1 / 440 / 5000 / 100000 frames, 3.80 dB): layout 7 at 16 or 24 CTAs per SM
+//   bf16: 45.2 / 84.2 / 190.8 / 3067, (1,1,0,0) 45.9 / 97.2 / 478.5 / 11184; min-sum 34.0 / 54.3 / 175.5 / 2607 against 38.3 /
+//         68.9 / 362.8 / 7348; with clips 46.4 / 87.3 / 209.8 / 4138 against 50.5 / 108.8 / 522.4 / 13509
+//   fp16: 41.9 / 78.2 / 186.3 / 3140, (1,1,0,0) 44.2 / 98.6 / 457.6 / 11299
+//   fp32: 43.2 / 80.1 / 188.7 / 2631, layout 1 43.4 / 92.2 / 289.0 / 5677
+static const QcDefault qc_r45k1_default[] = {
+    {32, 18, STORE_BF16, -1, 0, 1, 1, 16, 7},
+    {32, 18, STORE_FP16, -1, 0, 1, 1, 16, 7},
+    {32, 18, STORE_FP32, -1, 0, 1, 1, 24, 7},
+};
+LDPC_QC_DEFAULTS(qc_r45k1_default)
