@@ -220,7 +220,8 @@ int64_t ldpc_launch_param_bytes(const ldpc_handle* h);
  * d_llr [n_frames][N-P] fp32 (device memory) into device buffers d_post [n_frames][N], d_iters,
  * d_synd_fail, d_bit_errors (each may be NULL), on `stream` (a cudaStream_t; NULL = the legacy
  * default stream), and returns the tallies in *out.  Same decoder and results as ldpc_decode_llr
- * (the general file-order kernel); no cudaMalloc, cudaFree or host allocation.
+ * (the QC kernel for a matrix with that structure and d_llr 16-byte aligned, else the general file-order
+ * kernel); no cudaMalloc, cudaFree or host allocation.
  *
  * Its scratch (code tables, check messages, claim counter, tallies) is one static device array of
  * LDPC_STATIC_SCRATCH_BYTES that every GPU loading the library holds until exit.  A matrix needing

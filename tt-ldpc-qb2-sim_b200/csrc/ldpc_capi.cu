@@ -127,55 +127,62 @@ struct ldpc_handle {
     int stage_next = 0;
 };
 
-static int detect_qc(ldpc_handle* h) {
+namespace ldpcb200 {
+bool qc_structure(const int32_t* rows, int N, int M, int P, int dmax, QcStructure* out) {
     // 12 layers of Z rows; layers 0-3 of degree 3, layers 4-11 of one degree D; each edge of a layer
     // is a circulant: column(j) = blk*Z + ((j + s) mod Z) for every row j of the layer, and the
     // edges of a layer sit in distinct blocks (then the layer's rows share no column).
-    if (h->M % QC_LAYERS) return 0;
-    const int Z = h->M / QC_LAYERS;
-    if (Z < 32 || (Z & (Z - 1)) || h->N % Z || h->P % Z) return 0;
+    if (M % QC_LAYERS) return false;
+    const int Z = M / QC_LAYERS;
+    if (Z < 32 || (Z & (Z - 1)) || N % Z || P % Z) return false;
     int D = -1;
     for (int l = 0; l < QC_LAYERS; ++l) {
-        const int32_t* r0 = &h->rows[(size_t)(l * Z) * h->dmax];
+        const int32_t* r0 = &rows[(size_t)(l * Z) * dmax];
         int d = 0;
-        while (d < h->dmax && r0[d] >= 0) ++d;
-        if (l < 4 && d != QC_DEG_LOW) return 0;
+        while (d < dmax && r0[d] >= 0) ++d;
+        if (l < 4 && d != QC_DEG_LOW) return false;
         if (l >= 4) {
             if (D < 0) D = d;
-            if (d != D) return 0;
+            if (d != D) return false;
         }
-        if (d > QC_DMAX) return 0;
-        std::vector<int> blks;
+        if (d > QC_DMAX) return false;
         for (int e = 0; e < d; ++e) {
             const int c0 = r0[e];
             const int blk = c0 / Z, s = c0 % Z;
-            blks.push_back(blk);
-            for (int j = 0; j < Z; ++j) {
-                const int32_t* rj = &h->rows[(size_t)(l * Z + j) * h->dmax];
-                if (rj[e] != blk * Z + ((j + s) & (Z - 1))) return 0;
-            }
-            h->blk_off[l][e] = blk * Z;
-            h->shift[l][e] = s;
+            for (int j = 0; j < Z; ++j)
+                if (rows[(size_t)(l * Z + j) * dmax + e] != blk * Z + ((j + s) & (Z - 1))) return false;
+            out->blk_off[l][e] = blk * Z;
+            out->shift[l][e] = s;
+            for (int f = 0; f < e; ++f)
+                if (out->blk_off[l][f] == blk * Z) return false;
         }
-        for (int j = 0; j < Z; ++j) {
-            const int32_t* rj = &h->rows[(size_t)(l * Z + j) * h->dmax];
-            if (d < h->dmax && rj[d] >= 0) return 0;
-        }
-        std::sort(blks.begin(), blks.end());
-        if (std::adjacent_find(blks.begin(), blks.end()) != blks.end()) return 0;
+        for (int j = 0; j < Z; ++j)
+            if (d < dmax && rows[(size_t)(l * Z + j) * dmax + d] >= 0) return false;
     }
-    h->Z = Z;
-    h->D = D;
-    // a code whose descriptors some kernels have compiled in (layout 5)
-    h->fix = -1;
-    for (int i = 0; i < QC_FIXED_COUNT && h->fix < 0; ++i) {
+    out->Z = Z;
+    out->D = D;
+    // a code whose descriptors some kernels have compiled in (layouts 5 and 6)
+    out->fix = -1;
+    for (int i = 0; i < QC_FIXED_COUNT && out->fix < 0; ++i) {
         const QcFixedTable& t = kQcFixedHost[i];
         bool same = t.Z == Z && t.D == D;
         for (int l = 0; l < QC_LAYERS && same; ++l)
             for (int e = 0; e < (l < 4 ? QC_DEG_LOW : D) && same; ++e)
-                same = t.blk_off[l][e] == h->blk_off[l][e] && t.shift[l][e] == h->shift[l][e];
-        if (same) h->fix = i;
+                same = t.blk_off[l][e] == out->blk_off[l][e] && t.shift[l][e] == out->shift[l][e];
+        if (same) out->fix = i;
     }
+    return true;
+}
+}  // namespace ldpcb200
+
+static int detect_qc(ldpc_handle* h) {
+    QcStructure s = {};
+    if (!qc_structure(h->rows.data(), h->N, h->M, h->P, h->dmax, &s)) return 0;
+    h->Z = s.Z;
+    h->D = s.D;
+    h->fix = s.fix;
+    memcpy(h->blk_off, s.blk_off, sizeof h->blk_off);
+    memcpy(h->shift, s.shift, sizeof h->shift);
     return 1;
 }
 
@@ -349,39 +356,48 @@ static const void* find_shape(const ldpc_handle* h, int storage, int algo, int c
     return find_qc(QcKey{h->Z, h->D, R, F, storage, algo, clip, ext, B, G});
 }
 
-static bool shape_in_scratch(int G) { return G == 1 || G == 5 || G == 7; }  // messages in global memory
-
 // The default shape of a numerics variant for a call of n frames: the first line of the defaults that
 // applies (QcDefault), else one row per thread and one frame per CTA with messages in registers when that is
 // built, else the first shape built for it (e.g. the global-message kernel of a K = 16384 code).
 // scratch = false leaves out the lines that need a message scratch.
-static bool default_shape(const ldpc_handle* h, int storage, int algo, int clip, int ext, uint32_t n, bool scratch,
-                          int s[4]) {
+namespace ldpcb200 {
+const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4]) {
+    auto built = [&](int R, int F, int B, int G) -> const void* {
+        if ((G == 5 || G == 6) && fix < 0) return nullptr;  // compiled-in descriptors of another code
+        return find_qc(QcKey{Z, D, R, F, storage, algo, clip, ext, B, G});
+    };
     for (int own = 1; own >= 0; --own)
         for (const QcDefaults* t = qc_defaults(); t; t = t->next)
             for (int i = 0; i < t->count; ++i) {
                 const QcDefault& d = t->entries[i];
-                if (d.Z != h->Z || d.D != h->D || d.mode != storage || d.algo != (own ? algo : -1) || n < d.min_frames ||
-                    (!scratch && shape_in_scratch(d.G)) ||
-                    !find_shape(h, storage, algo, clip, ext, d.R, d.F, d.B, d.G))
+                if (d.Z != Z || d.D != D || d.mode != storage || d.algo != (own ? algo : -1) || n < d.min_frames ||
+                    (!scratch && qc_shape_in_scratch(d.G)))
                     continue;
-                s[0] = d.R; s[1] = d.F; s[2] = d.B; s[3] = d.G;
-                return true;
+                if (const void* fn = built(d.R, d.F, d.B, d.G)) {
+                    s[0] = d.R; s[1] = d.F; s[2] = d.B; s[3] = d.G;
+                    return fn;
+                }
             }
-    if (find_shape(h, storage, algo, clip, ext, 1, 1, 0, 0)) {
+    if (const void* fn = built(1, 1, 0, 0)) {
         s[0] = 1; s[1] = 1; s[2] = 0; s[3] = 0;
-        return true;
+        return fn;
     }
     for (const QcTable* t = qc_tables(); t; t = t->next)
         for (int i = 0; i < t->count; ++i) {
             const QcKey& k = t->entries[i].key;
-            if (k.Z == h->Z && k.D == h->D && k.mode == storage && k.algo == algo && k.clip == clip && k.ext == ext &&
-                ((k.G != 5 && k.G != 6) || h->fix >= 0)) {
+            if (k.Z == Z && k.D == D && k.mode == storage && k.algo == algo && k.clip == clip && k.ext == ext &&
+                ((k.G != 5 && k.G != 6) || fix >= 0)) {
                 s[0] = k.R; s[1] = k.F; s[2] = k.B; s[3] = k.G;
-                return true;
+                return t->entries[i].fn;
             }
         }
-    return false;
+    return nullptr;
+}
+}  // namespace ldpcb200
+
+static bool default_shape(const ldpc_handle* h, int storage, int algo, int clip, int ext, uint32_t n, bool scratch,
+                          int s[4]) {
+    return qc_default(h->Z, h->D, h->fix, storage, algo, clip, ext, n, scratch, s) != nullptr;
 }
 
 static bool default_shape_exists(const ldpc_handle* h, int storage, int algo) {
@@ -578,6 +594,25 @@ static int check_params(const ldpc_handle* h, const ldpc_run_params* p) {
     return 0;
 }
 
+namespace ldpcb200 {
+// The global-message layout keeps edges in pairs: odd degrees padded.
+void qc_message_layout(QcParams* qp, int Z, int D) {
+    int32_t off = 0;
+    for (int l = 0; l < QC_LAYERS; ++l) {
+        qp->layer_off[l] = off;
+        off += Z * (((l < 4 ? QC_DEG_LOW : D) + 1) & ~1);
+    }
+    qp->slot_elems = off;
+}
+// The kernel's shared memory: L slots, hard-decision words, [16-byte aligned] offset table (G = 2).
+size_t qc_smem_bytes(int N, int Z, int D, int R, int F, int G, int storage) {
+    const size_t esz = storage == LDPC_STORE_BF16 ? 2 : 4;
+    size_t smem = (size_t)F * ((N + 7) & ~7) * esz + (size_t)F * (N / 32) * 4;
+    if (G == 2) smem = ((smem + 15) & ~(size_t)15) + (size_t)(Z / R) * (QC_DEG_LOW * 4 + D * 8) * 4;
+    return smem;
+}
+}  // namespace ldpcb200
+
 // A prepared QC launch: kernel, grid, block, dynamic shared memory and its parameter block.
 struct QcLaunch {
     const void* fn = nullptr;
@@ -623,11 +658,11 @@ static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32
     const void* fn = lookup(wrow ? ALGO_WROW : p->algo);
     if (!fn) return LDPC_ENOTSUP;  // the caller falls back to the general kernel
     int rc = prepare_qc_shape(h, p, fn, sh, wrow, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, grid_frac, out);
-    if (rc == LDPC_ENOMEM && !chosen && shape_in_scratch(sh[3])) {
+    if (rc == LDPC_ENOMEM && !chosen && qc_shape_in_scratch(sh[3])) {
         // no memory for a default shape's message scratch: the default without one, where there is one
         scratch = false;
         fn = lookup(wrow ? ALGO_WROW : p->algo);
-        if (fn && !shape_in_scratch(sh[3]))
+        if (fn && !qc_shape_in_scratch(sh[3]))
             rc = prepare_qc_shape(h, p, fn, sh, wrow, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, grid_frac, out);
     }
     return rc;
@@ -702,18 +737,9 @@ static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void
         qp.n_info = h->N - h->M;
     }
     const int T = h->Z / R;
-    int32_t off = 0;
-    for (int l = 0; l < QC_LAYERS; ++l) {
-        qp.layer_off[l] = off;  // the global-message layout keeps edges in pairs: odd degrees padded
-        off += h->Z * (((l < 4 ? QC_DEG_LOW : h->D) + 1) & ~1);
-    }
-    qp.slot_elems = off;
-    const size_t esz = p->storage == LDPC_STORE_BF16 ? 2 : 4;
-    const size_t lstride = (size_t)((h->N + 7) & ~7);
-    // the kernel's layout: L slots, hard-decision words, [16-byte aligned] offset table (G = 2), weights
-    size_t smem = (size_t)F * lstride * esz + (size_t)F * (h->N / 32) * 4;
-    if (G == 2 || p->algo == LDPC_ALGO_WAMIN) smem = (smem + 15) & ~(size_t)15;
-    if (G == 2) smem += (size_t)T * (QC_DEG_LOW * 4 + h->D * 8) * 4;
+    qc_message_layout(&qp, h->Z, h->D);
+    size_t smem = qc_smem_bytes(h->N, h->Z, h->D, R, F, G, p->storage);
+    if (p->algo == LDPC_ALGO_WAMIN) smem = (smem + 15) & ~(size_t)15;
     if (p->algo == LDPC_ALGO_WAMIN) smem += (size_t)qp.w_iters * qp.w_slots * sizeof(float2);
     if (smem > 48 * 1024) CU(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
@@ -727,7 +753,7 @@ static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void
     out->block = T;
     out->smem = smem;
     if (grid == 0) return 0;
-    if (shape_in_scratch(G)) {
+    if (qc_shape_in_scratch(G)) {
         int rc;
         const size_t rsz = p->storage == LDPC_STORE_FP32 ? 4 : 2;
         if ((rc = ensure_cap(&h->d_rmsg, &h->rmsg_cap, grid * F * (size_t)qp.slot_elems * rsz))) return rc;

@@ -80,6 +80,18 @@ struct QcParams {
     int32_t circ_sfpu;
 };
 
+// Host side (ldpc_capi.cu).  The quasi-cyclic structure of a row table, found without allocating; the default
+// kernel and shape (QcDefault) of a call; the message layout and shared memory a launch needs.
+struct QcStructure {
+    int Z, D;
+    int fix;  // index of the compiled-in descriptors that are exactly these, or -1
+    int32_t blk_off[QC_LAYERS][QC_DMAX], shift[QC_LAYERS][QC_DMAX];
+};
+bool qc_structure(const int32_t* rows, int N, int M, int P, int dmax, QcStructure* out);
+const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4]);
+void qc_message_layout(QcParams* qp, int Z, int D);
+size_t qc_smem_bytes(int N, int Z, int D, int R, int F, int G, int storage);
+
 enum QcStop : int { QC_STOP_SYNDROME = 0, QC_STOP_GENIE = 1 };
 
 // Slot of edge e of layer l in a per-iteration row of the weight table: layers 0-3 (degree 3) first.

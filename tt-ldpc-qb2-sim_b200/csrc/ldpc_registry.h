@@ -50,6 +50,8 @@ struct QcDefaults {
 void register_qc_defaults(QcDefaults* t);
 const QcDefaults* qc_defaults();
 
+inline bool qc_shape_in_scratch(int G) { return G == 1 || G == 5 || G == 7; }  // messages in global memory
+
 // Linked at static-initialisation time by each instantiation unit.
 void register_qc_table(QcTable* t);
 const QcTable* qc_tables();

@@ -55,6 +55,16 @@ static const QcEntry qc_k16[] = {
     LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 2, 2),
     LDPC_QC_ENTRY_GF_NAN(512, 18, 1, 1, STORE_BF16, ALGO_NMS, true, 2, 2),
     LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 2, 2),
+    // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
+    LDPC_QC_ENTRY_GF(2048, 6, 4, 1, STORE_FP16, ALGO_AMIN, true, true, 0, 0),
+    LDPC_QC_ENTRY_G(2048, 6, 4, 1, STORE_FP32, ALGO_AMIN, true, true, 0),
+    LDPC_QC_ENTRY_GF(2048, 6, 4, 1, STORE_BF16, ALGO_NMS, true, true, 0, 0),
+    LDPC_QC_ENTRY_GF(1024, 10, 2, 1, STORE_FP16, ALGO_AMIN, true, true, 2, 1),
+    LDPC_QC_ENTRY_G(1024, 10, 2, 1, STORE_FP32, ALGO_AMIN, true, true, 0),
+    LDPC_QC_ENTRY_GF(1024, 10, 2, 1, STORE_BF16, ALGO_NMS, true, true, 0, 1),
+    LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 2, 2),
+    LDPC_QC_ENTRY_G(512, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 0),
+    LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_BF16, ALGO_NMS, true, true, 2, 2),
 };
 LDPC_QC_REGISTER(qc_k16)
 

@@ -96,6 +96,9 @@ static const QcEntry qc_r12k1[] = {
     LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 8, 5),
     LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_BF16, ALGO_NMS, false, true, 8, 5),
     LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 8, 5),
+    // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 6, 5),
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 5, 5),
 };
 LDPC_QC_REGISTER(qc_r12k1)
 

@@ -38,6 +38,9 @@ static const QcEntry qc_r12k4[] = {
     LDPC_QC_ENTRY_RF(512, 6, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 2, 6),
     LDPC_QC_ENTRY_RF(512, 6, 1, 1, STORE_BF16, ALGO_NMS, false, true, 2, 6),
     LDPC_QC_ENTRY_RF(512, 6, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 2, 6),
+    // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
+    LDPC_QC_ENTRY_RF(512, 6, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 2, 6),
+    LDPC_QC_ENTRY_RF(512, 6, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 1, 6),
 };
 LDPC_QC_REGISTER(qc_r12k4)
 

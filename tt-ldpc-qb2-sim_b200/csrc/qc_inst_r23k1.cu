@@ -47,6 +47,10 @@ static const QcEntry qc_r23k1[] = {
     LDPC_QC_ENTRY_RF(64, 10, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 0, 8),
     LDPC_QC_ENTRY_RF(64, 10, 1, 1, STORE_BF16, ALGO_NMS, false, true, 0, 8),
     LDPC_QC_ENTRY_RF(64, 10, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 0, 8),
+    // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
+    LDPC_QC_ENTRY_OT(64, 10, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 0),
+    LDPC_QC_ENTRY_GR(64, 10, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 0),
+    LDPC_QC_ENTRY_OT(64, 10, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 0),
 };
 LDPC_QC_REGISTER(qc_r23k1)
 

@@ -34,6 +34,9 @@ static const QcEntry qc_r23k4[] = {
     LDPC_QC_ENTRY_RF(256, 10, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 2, 7),
     LDPC_QC_ENTRY_RF(256, 10, 1, 1, STORE_BF16, ALGO_NMS, false, true, 2, 7),
     LDPC_QC_ENTRY_RF(256, 10, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 2, 7),
+    // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
+    LDPC_QC_ENTRY_RF(256, 10, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 3, 7),
+    LDPC_QC_ENTRY_RF(256, 10, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 2, 7),
 };
 LDPC_QC_REGISTER(qc_r23k4)
 

@@ -57,6 +57,9 @@ static const QcEntry qc_r45k1[] = {
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 16),
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_NMS, false, true, 16),
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 16),
+    // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 16),
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 24),
 };
 LDPC_QC_REGISTER(qc_r45k1)
 

@@ -80,6 +80,9 @@ static const QcEntry qc_r45k4[] = {
     LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, false, 6),
     LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_BF16, ALGO_NMS, false, true, 6),
     LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_BF16, ALGO_AMIN, true, true, 6),
+    // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
+    LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 6),
+    LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 6),
 };
 LDPC_QC_REGISTER(qc_r45k4)
 
