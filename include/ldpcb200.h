@@ -313,6 +313,12 @@ int ldpc_wdec_backward(ldpc_handle* h, const ldpc_wdec_config* c, int64_t n_fram
                        const void* d_beta, const void* d_grad_post, void* d_grad_alpha, void* d_grad_beta,
                        void* d_grad_llr, void* d_workspace, void* stream);
 
+/* The training losses' pass over the posteriors: d_out[r] = sum over i of softplus(-d_x[r][i]) (softplus(y) =
+ * log(1 + e^y)), r < rows, i < n, and its adjoint d_gx[r][i] = -d_g[r] sigmoid(-d_x[r][i]).  float arrays in
+ * device memory of the current device, queued on the stream; d_x and d_gx 16-byte aligned, n a multiple of 4. */
+int ldpc_softplus_rows(const float* d_x, int64_t rows, int32_t n, float* d_out, void* stream);
+int ldpc_softplus_rows_grad(const float* d_x, const float* d_g, int64_t rows, int32_t n, float* d_gx, void* stream);
+
 /* A batch of codes on one device decoded by one CUDA graph launch (the mixed-code workload).  The
  * reference runs one code per process (run_simulation.py:164-193); this has no counterpart there.
  * Every handle must have the QC structure. */

@@ -16,6 +16,7 @@
 
 #include "../../include/ldpcb200.h"
 #include "ldpc_general.cuh"
+#include "ldpc_loss.cuh"
 #include "ldpc_qc.cuh"
 #include "ldpc_registry.h"
 #include "ldpc_weighted.cuh"
@@ -1485,5 +1486,32 @@ extern "C" int ldpc_wdec_backward(ldpc_handle* h, const ldpc_wdec_config* c, int
     wworkspace(&p, d_ws, rb);
     if ((rc = weighted_launch(p, h->Z, h->D, rb, false, h->n_sm, s, g_err))) return rc;
     h->launches += n ? 1 : 0;
+    return 0;
+}
+
+// ----------------------------------------------------------------------------- training losses
+static int loss_check(const void* a, const void* b, int64_t rows, int32_t n, int* n_sm) {
+    if (rows < 0 || n < 4 || n % 4) return fail(LDPC_EINVAL, "rows %lld x %d: n must be a positive multiple of 4", (long long)rows, n);
+    if (rows && (!a || !b)) return fail(LDPC_EINVAL, "NULL device pointer");
+    if (reinterpret_cast<uintptr_t>(a) % 16) return fail(LDPC_EINVAL, "the rows must be 16-byte aligned");
+    int dev = 0;
+    CU(cudaGetDevice(&dev));
+    CU(cudaDeviceGetAttribute(n_sm, cudaDevAttrMultiProcessorCount, dev));
+    return 0;
+}
+
+extern "C" int ldpc_softplus_rows(const float* d_x, int64_t rows, int32_t n, float* d_out, void* stream) {
+    int rc, n_sm = 0;
+    if ((rc = loss_check(d_x, d_out, rows, n, &n_sm))) return rc;
+    if (rows) CU(softplus_rows(d_x, (uint64_t)rows, n, d_out, n_sm, static_cast<cudaStream_t>(stream)));
+    return 0;
+}
+
+extern "C" int ldpc_softplus_rows_grad(const float* d_x, const float* d_g, int64_t rows, int32_t n, float* d_gx, void* stream) {
+    int rc, n_sm = 0;
+    if ((rc = loss_check(d_x, d_g, rows, n, &n_sm))) return rc;
+    if (rows && !d_gx) return fail(LDPC_EINVAL, "NULL device pointer");
+    if (reinterpret_cast<uintptr_t>(d_gx) % 16) return fail(LDPC_EINVAL, "the rows must be 16-byte aligned");
+    if (rows) CU(softplus_rows_grad(d_x, d_g, (uint64_t)rows, n, d_gx, n_sm, static_cast<cudaStream_t>(stream)));
     return 0;
 }

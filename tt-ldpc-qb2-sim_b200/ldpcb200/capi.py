@@ -29,6 +29,7 @@ EXPORTS = ("ldpc_create", "ldpc_destroy", "ldpc_kernel_kind", "ldpc_run_chunk", 
            "ldpc_set_launch_shape", "ldpc_list_shapes", "ldpc_list_shapes_algo", "ldpc_set_weights",
            "ldpc_set_circulant",
            "ldpc_wdec_workspace_bytes", "ldpc_wdec_forward", "ldpc_wdec_backward",
+           "ldpc_softplus_rows", "ldpc_softplus_rows_grad",
            "ldpc_launch_count", "ldpc_batch_create", "ldpc_batch_destroy", "ldpc_batch_run",
            "ldpc_batch_graph_builds", "ldpc_batch_set_order",
            "ldpc_launch_param_bytes", "ldpc_decode_llr_static", "ldpc_row_schedule", "ldpc_step_schedule",
@@ -128,6 +129,8 @@ def load(path: str = LIB_PATH):
                                     C.c_void_p, C.c_void_p, C.c_void_p]
     L.ldpc_wdec_backward.argtypes = [C.c_void_p, P(WdecConfig), C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
                                      C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
+    L.ldpc_softplus_rows.argtypes = [C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]
+    L.ldpc_softplus_rows_grad.argtypes = [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p]
     L.ldpc_launch_count.argtypes = [C.c_void_p]
     L.ldpc_launch_count.restype = C.c_int64
     L.ldpc_launch_param_bytes.argtypes = [C.c_void_p]

@@ -6,8 +6,9 @@ Approximate-Min* magnitude the plain decoder would send on edge e (ldpc_decoder_
 the reference), t the iteration and c the protograph edge class of the edge (one class per edge of
 the AR4JA base matrix, ar4ja.QcCode.edge_class).  It runs exactly T iterations (no early stop), so
 it can be differentiated; the forward and the adjoint are hand-written CUDA kernels
-(csrc/weighted.cu) behind ``WeightedFn``, and the adjoint recomputes each segment of ``ckpt_every``
-iterations from an activation checkpoint.  With alpha = 1 and beta = 0 the forward pass gives the
+(csrc/weighted.cu) behind ``WeightedFn``.  The forward keeps the rows of as many of the last
+iterations as fit the memory that checkpoints every ``ckpt_every`` iterations would take; the adjoint
+runs the iterations before them again.  With alpha = 1 and beta = 0 the forward pass gives the
 plain fp32 decoder's values bit for bit.
 
 Training (``train``) draws its frames from the simulator's own channel (Philox + Box-Muller AWGN,
@@ -179,12 +180,58 @@ class WeightedDecoder(torch.nn.Module):
         self.dec.close()
 
 
+class SoftplusRows(torch.autograd.Function):
+    """softplus(-x).sum(-1) in one pass over x (csrc/loss.cu), and its gradient in one more."""
+
+    @staticmethod
+    def forward(ctx, x):
+        ctx.save_for_backward(x)
+        out = torch.empty(x.shape[:-1], dtype=x.dtype, device=x.device)
+        with torch.cuda.device(x.device):
+            s = torch.cuda.current_stream(x.device).cuda_stream
+            capi._check(capi.load().ldpc_softplus_rows(x.data_ptr(), out.numel(), x.shape[-1], out.data_ptr(), s or None))
+        return out
+
+    @staticmethod
+    def backward(ctx, g):
+        (x,) = ctx.saved_tensors
+        # a gradient that is itself differentiated, or one of a batch of gradients (it has no storage)
+        if torch.is_grad_enabled() or not _one_pass(x) or not torch._C._has_storage(g):
+            return -g.unsqueeze(-1) * torch.sigmoid(-x)
+        g = g.contiguous()
+        gx = torch.empty_like(x)
+        with torch.cuda.device(x.device):
+            s = torch.cuda.current_stream(x.device).cuda_stream
+            capi._check(capi.load().ldpc_softplus_rows_grad(x.data_ptr(), g.data_ptr(), g.numel(), x.shape[-1],
+                                                            gx.data_ptr(), s or None))
+        return gx
+
+
+def _one_pass(x: torch.Tensor) -> bool:
+    """Whether softplus(-x).sum(-1) runs on the one-pass kernels: plain contiguous float32 CUDA rows, and
+    nothing that looks into the operations (function transforms, forward-mode differentiation, tracing,
+    compilation, dispatch modes) is active; everything else takes the library's operations."""
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and not torch._C._are_functorch_transforms_active()
+            and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing()
+            and not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._len_torch_function_stack() == 0 and x.is_cuda and x.dtype == torch.float32 and x.dim() > 0
+            and x.numel() > 0 and x.shape[-1] % 4 == 0 and x.shape[-1] < 2 ** 31 and x.is_contiguous()
+            and not x.is_neg() and x.data_ptr() % 16 == 0)
+
+
+def softplus_rows(post: torch.Tensor) -> torch.Tensor:
+    """softplus(-post) summed over the last dimension."""
+    return SoftplusRows.apply(post) if _one_pass(post) else torch.nn.functional.softplus(-post).sum(-1)
+
+
 def bce_allzero(post: torch.Tensor, iters: Optional[Tuple[int, int]] = None) -> torch.Tensor:
     """Binary cross-entropy of posterior LLRs (positive = bit 0) against the all-zero codeword, over
     all iterations' posteriors [T][B][N] or only those of iterations iters[0]..iters[1] (1-based)."""
     if iters is not None:
         post = post[iters[0] - 1:iters[1]]
-    return torch.nn.functional.softplus(-post).mean()
+    if not _one_pass(post):
+        return torch.nn.functional.softplus(-post).mean()
+    return softplus_rows(post).mean() / post.shape[-1]
 
 
 def stop_loss(post: torch.Tensor) -> torch.Tensor:
@@ -194,8 +241,9 @@ def stop_loss(post: torch.Tensor) -> torch.Tensor:
     iterations of 1 - exp(-S) estimates the expected fraction of the T iterations a frame still runs,
     so its gradient goes to the frames about to converge; the mean bit BCE is added so frames far from
     convergence still pull the posteriors the right way."""
-    S = torch.nn.functional.softplus(-post).sum(-1)  # [T][B]
-    return (1.0 - torch.exp(-S)).mean() + torch.nn.functional.softplus(-post).mean()
+    S = softplus_rows(post)  # [T][B]
+    bce = S.mean() / post.shape[-1] if _one_pass(post) else torch.nn.functional.softplus(-post).mean()
+    return (-torch.expm1(-S)).mean() + bce  # 1 - exp(-S) without its cancellation for small S
 
 
 LOSSES = {"bce": lambda post, iters: bce_allzero(post, iters), "stop": lambda post, iters: stop_loss(post)}
