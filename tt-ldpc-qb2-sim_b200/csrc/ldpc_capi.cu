@@ -88,12 +88,23 @@ struct ldpc_handle {
     bool gen_built = false;
     // general structure (device)
     GeneralCode gen{};
-    // device scratch
+    // device scratch: one block (d_io), the counters first, so that one memset clears them, the tally last of
+    // them and followed by the outputs of a small ldpc_decode_llr call, so that one copy brings both back
+    unsigned char* d_io = nullptr;
+    unsigned int* d_work = nullptr;         // [16]
+    unsigned long long* d_hist = nullptr;   // [hist_bins]
+    unsigned long long* d_snr = nullptr;    // [4][SNR_BINS]
     unsigned long long* d_tally = nullptr;  // [TALLY_WORDS]
-    unsigned int* d_work = nullptr;
-    unsigned long long* d_hist = nullptr;
-    int hist_bins = 0;
-    unsigned long long* d_snr = nullptr;  // [4][SNR_BINS]
+    static constexpr int hist_bins = 1024;
+    static constexpr size_t kCounterBytes = 64 + hist_bins * 8 + 4 * SNR_BINS * 8 + TALLY_WORDS * 8;
+    static constexpr size_t kTallyOff = kCounterBytes - TALLY_WORDS * 8;
+    // LLRs (as fp32) and outputs of a small call, at most this much each; then the same LLRs as bf16
+    static constexpr size_t kSmallBytes = 1u << 20;
+    static constexpr size_t kSmallLlr = (kCounterBytes + kSmallBytes + 255) / 256 * 256;
+    static constexpr size_t kSmallLlr16 = kSmallLlr + kSmallBytes;
+    static constexpr size_t kIoBytes = kSmallLlr16 + kSmallBytes / 2;
+    unsigned char* h_small = nullptr;  // pinned, on first use: tally and outputs, then LLRs
+    static constexpr size_t kSmallHostLlr = (TALLY_WORDS * 8 + kSmallBytes + 255) / 256 * 256;
     float* d_llr = nullptr;
     size_t llr_cap = 0;
     float* d_post = nullptr;
@@ -214,10 +225,7 @@ extern "C" void ldpc_destroy(ldpc_handle* h) {
     if (!h) return;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    cudaFree(h->d_tally);
-    cudaFree(h->d_work);
-    cudaFree(h->d_hist);
-    cudaFree(h->d_snr);
+    cudaFree(h->d_io);
     cudaFree(h->d_llr);
     cudaFree(h->d_post);
     cudaFree(h->d_frame_out);
@@ -226,6 +234,7 @@ extern "C" void ldpc_destroy(ldpc_handle* h) {
     cudaFree(h->d_wtab_row);
     free_general(&h->gen);
     if (h->h_tally) cudaFreeHost(h->h_tally);
+    if (h->h_small) cudaFreeHost(h->h_small);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
@@ -274,21 +283,26 @@ extern "C" int ldpc_create(const ldpc_matrix* m, int device, ldpc_handle** out) 
     int rc = 0;
     auto bail = [&](int code) { ldpc_destroy(h); return code; };
     if (cudaSetDevice(device) != cudaSuccess) return bail(fail(LDPC_ENODEV, "cudaSetDevice(%d) failed", device));
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return bail(fail(LDPC_ENODEV, "no device properties"));
-    if (prop.major < 10) return bail(fail(LDPC_ENODEV, "device %s (sm_%d%d) is not sm_100", prop.name, prop.major, prop.minor));
-    h->n_sm = prop.multiProcessorCount;
+    // (cudaGetDeviceProperties takes milliseconds; these two attributes microseconds)
+    int major = 0;
+    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&h->n_sm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+        return bail(fail(LDPC_ENODEV, "no device properties"));
+    if (major < 10) {
+        cudaDeviceProp prop;
+        if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return bail(fail(LDPC_ENODEV, "no device properties"));
+        return bail(fail(LDPC_ENODEV, "device %s (sm_%d%d) is not sm_100", prop.name, prop.major, prop.minor));
+    }
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
         return bail(fail(LDPC_EIO, "stream/event creation failed"));
-    if (cudaMalloc(&h->d_tally, TALLY_WORDS * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&h->d_work, 64) != cudaSuccess ||
+    if (cudaMalloc(&h->d_io, ldpc_handle::kIoBytes) != cudaSuccess ||
         cudaMallocHost(&h->h_tally, TALLY_WORDS * sizeof(unsigned long long)) != cudaSuccess)
         return bail(fail(LDPC_ENOMEM, "device allocation failed"));
-    h->hist_bins = 1024;
-    if (cudaMalloc(&h->d_hist, h->hist_bins * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&h->d_snr, 4 * SNR_BINS * sizeof(unsigned long long)) != cudaSuccess)
-        return bail(fail(LDPC_ENOMEM, "device allocation failed"));
+    h->d_work = reinterpret_cast<unsigned int*>(h->d_io);
+    h->d_hist = reinterpret_cast<unsigned long long*>(h->d_io + 64);
+    h->d_snr = h->d_hist + h->hist_bins;
+    h->d_tally = reinterpret_cast<unsigned long long*>(h->d_io + ldpc_handle::kTallyOff);
     if (detect_qc(h) && h->N - h->P > 0 && ((h->N - h->P) % 32) == 0) {
         h->kind = LDPC_KERNEL_QC;
     } else {
@@ -775,10 +789,24 @@ static int launch_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32_
 }
 
 static int reset_counters(ldpc_handle* h) {
-    CU(cudaMemsetAsync(h->d_tally, 0, TALLY_WORDS * sizeof(unsigned long long), h->stream));
-    CU(cudaMemsetAsync(h->d_work, 0, 64, h->stream));
-    CU(cudaMemsetAsync(h->d_hist, 0, h->hist_bins * sizeof(unsigned long long), h->stream));
-    CU(cudaMemsetAsync(h->d_snr, 0, 4 * SNR_BINS * sizeof(unsigned long long), h->stream));
+    CU(cudaMemsetAsync(h->d_io, 0, ldpc_handle::kCounterBytes, h->stream));
+    return 0;
+}
+
+static int fill_tally(ldpc_handle* h, const unsigned long long* t, ldpc_tally* out) {
+    float ms = 0.0f;
+    CU(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
+    if (out) {
+        out->frames = t[T_FRAMES];
+        out->bit_errors = t[T_BIT_ERR];
+        out->frame_errors = t[T_FRAME_ERR];
+        out->iter_sum = t[T_ITER_SUM];
+        out->unconverged = t[T_UNCONVERGED];
+        out->max_iters = t[T_MAX_ITER];
+        out->kernel_ms = ms;
+        out->reserved1 = 0.0f;
+        out->bit_errors_sq = t[T_BIT_ERR_SQ];
+    }
     return 0;
 }
 
@@ -786,20 +814,7 @@ static int read_tally(ldpc_handle* h, ldpc_tally* out) {
     CU(cudaMemcpyAsync(h->h_tally, h->d_tally, TALLY_WORDS * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                        h->stream));
     CU(cudaStreamSynchronize(h->stream));
-    float ms = 0.0f;
-    CU(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
-    if (out) {
-        out->frames = h->h_tally[T_FRAMES];
-        out->bit_errors = h->h_tally[T_BIT_ERR];
-        out->frame_errors = h->h_tally[T_FRAME_ERR];
-        out->iter_sum = h->h_tally[T_ITER_SUM];
-        out->unconverged = h->h_tally[T_UNCONVERGED];
-        out->max_iters = h->h_tally[T_MAX_ITER];
-        out->kernel_ms = ms;
-        out->reserved1 = 0.0f;
-        out->bit_errors_sq = h->h_tally[T_BIT_ERR_SQ];
-    }
-    return 0;
+    return fill_tally(h, h->h_tally, out);
 }
 
 // Splits a request into launches of at most 2^31 frames (the kernel's claim counter is 32-bit).
@@ -911,10 +926,8 @@ class CopyPool {
 
 static void par_memcpy(void* dst, const void* src, size_t bytes) { CopyPool::get().copy(dst, src, bytes); }
 
-// Host -> device copy of `bytes` from a pageable array through the pinned ring, on the copy stream:
-// each piece waits for its slot's previous copy, is copied into the slot by host threads, then
-// copied to the device asynchronously, so the host fills one slot while others travel.
-static int stage_h2d(ldpc_handle* h, void* dst, const char* src, size_t bytes) {
+// The pinned ring's slots and events, on first use.
+static int stage_alloc(ldpc_handle* h) {
     for (int i = 0; i < ldpc_handle::kStageSlots; ++i) {
         if (!h->stage[i] && cudaMallocHost(&h->stage[i], ldpc_handle::kStageBytes) != cudaSuccess) {
             cudaGetLastError();
@@ -923,6 +936,15 @@ static int stage_h2d(ldpc_handle* h, void* dst, const char* src, size_t bytes) {
         if (!h->stage_ev[i] && cudaEventCreateWithFlags(&h->stage_ev[i], cudaEventDisableTiming) != cudaSuccess)
             return fail(LDPC_EIO, "staging event creation failed");
     }
+    return 0;
+}
+
+// Host -> device copy of `bytes` from a pageable array through the pinned ring, on the copy stream:
+// each piece waits for its slot's previous copy, is copied into the slot by host threads, then
+// copied to the device asynchronously, so the host fills one slot while others travel.
+static int stage_h2d(ldpc_handle* h, void* dst, const char* src, size_t bytes) {
+    int rc;
+    if ((rc = stage_alloc(h))) return rc;
     for (size_t done = 0; done < bytes;) {
         const size_t piece = std::min(ldpc_handle::kStageBytes, bytes - done);
         const int k = h->stage_next;
@@ -1016,6 +1038,95 @@ extern "C" int ldpc_run_chunk(ldpc_handle* h, const ldpc_run_params* p, ldpc_tal
     return read_tally(h, out);
 }
 
+// Memory the host may read and write itself (neither device memory nor an unknown kind).
+static bool host_memory(const void* p, bool* pageable = nullptr) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        a.type = cudaMemoryTypeUnregistered;
+    }
+    if (pageable) *pageable = a.type == cudaMemoryTypeUnregistered;
+    return a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost;
+}
+
+static int small_alloc(ldpc_handle* h) {
+    if (!h->h_small &&
+        cudaMallocHost(&h->h_small, ldpc_handle::kSmallHostLlr + ldpc_handle::kSmallBytes) != cudaSuccess) {
+        cudaGetLastError();
+        h->h_small = nullptr;
+        return fail(LDPC_ENOMEM, "pinned buffer allocation failed");
+    }
+    return 0;
+}
+
+// A call whose LLRs and outputs take at most kSmallBytes each: one stream, one pinned buffer, one copy each way
+// (the outputs follow the tally on the device), the caller's arrays read and written by the host.  One frame
+// r1/2 K=1024 fp32 with posteriors, whole call: 59 us, 113 with the copies of the large path (a second
+// stream, one copy per output into pageable memory); its first call on a handle 3 ms, 69 to 80 with the ring.
+static int decode_small(ldpc_handle* h, const ldpc_run_params* p, const void* llr, int elem, size_t n, float* post,
+                        int32_t* iters, int32_t* synd_fail, int32_t* bit_errors, ldpc_tally* out) {
+    using H = ldpc_handle;
+    int rc;
+    if ((rc = small_alloc(h))) return rc;
+    const size_t ntx = (size_t)(h->N - h->P), in_bytes = n * ntx * elem;
+    unsigned char* h_llr = h->h_small + H::kSmallHostLlr;
+    float* d_llr = reinterpret_cast<float*>(h->d_io + H::kSmallLlr);
+    uint16_t* d_llr16 = reinterpret_cast<uint16_t*>(h->d_io + H::kSmallLlr16);
+    memcpy(h_llr, llr, in_bytes);
+    CU(cudaMemcpyAsync(elem == 4 ? static_cast<void*>(d_llr) : static_cast<void*>(d_llr16), h_llr, in_bytes,
+                       cudaMemcpyHostToDevice, h->stream));
+    if (elem == 2) {
+        widen_bf16_kernel<<<(unsigned)std::min<size_t>((n * ntx + 2047) / 2048, h->n_sm * 4), 256, 0, h->stream>>>(
+            d_llr16, d_llr, n * ntx);
+        CU(cudaGetLastError());
+    }
+    int32_t* d_it = reinterpret_cast<int32_t*>(h->d_io + H::kCounterBytes);
+    int32_t *d_sf = d_it + n, *d_be = d_sf + n;
+    float* d_post = reinterpret_cast<float*>(d_be + n);
+    if ((rc = run_frames(h, p, true, n, d_llr, post ? d_post : nullptr, d_it, d_sf, d_be))) return rc;
+    const size_t post_bytes = post ? n * h->N * sizeof(float) : 0;
+    CU(cudaMemcpyAsync(h->h_small, h->d_tally, TALLY_WORDS * 8 + 3 * n * sizeof(int32_t) + post_bytes,
+                       cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaStreamSynchronize(h->stream));
+    const unsigned char* o = h->h_small + TALLY_WORDS * 8;
+    if (iters) memcpy(iters, o, n * sizeof(int32_t));
+    if (synd_fail) memcpy(synd_fail, o + n * sizeof(int32_t), n * sizeof(int32_t));
+    if (bit_errors) memcpy(bit_errors, o + 2 * n * sizeof(int32_t), n * sizeof(int32_t));
+    if (post) memcpy(post, o + 3 * n * sizeof(int32_t), post_bytes);
+    return fill_tally(h, reinterpret_cast<const unsigned long long*>(h->h_small), out);
+}
+
+// Device -> host copy into a pageable array through the pinned ring: while the host copies one piece out of its
+// slot (threads share the work, and the page faults of a fresh array), the next piece travels.
+static int unstage_d2h(ldpc_handle* h, char* dst, const char* src, size_t bytes) {
+    int rc;
+    if ((rc = stage_alloc(h))) return rc;
+    const size_t piece = std::min<size_t>(ldpc_handle::kStageBytes, std::max<size_t>(1u << 20, bytes / 8));
+    size_t sent = 0, got = 0;
+    int first = h->stage_next, inflight = 0;
+    while (got < bytes) {
+        while (inflight < ldpc_handle::kStageSlots && sent < bytes) {
+            const int k = h->stage_next;
+            h->stage_next = (k + 1) % ldpc_handle::kStageSlots;
+            if (h->stage_busy[k]) CU(cudaEventSynchronize(h->stage_ev[k]));
+            const size_t b = std::min(piece, bytes - sent);
+            CU(cudaMemcpyAsync(h->stage[k], src + sent, b, cudaMemcpyDeviceToHost, h->stream));
+            CU(cudaEventRecord(h->stage_ev[k], h->stream));
+            h->stage_busy[k] = true;
+            sent += b;
+            ++inflight;
+        }
+        const size_t b = std::min(piece, bytes - got);
+        CU(cudaEventSynchronize(h->stage_ev[first]));
+        par_memcpy(dst + got, h->stage[first], b);
+        h->stage_busy[first] = false;
+        first = (first + 1) % ldpc_handle::kStageSlots;
+        --inflight;
+        got += b;
+    }
+    return 0;
+}
+
 // ldpc_decode_llr and ldpc_decode_llr_bf16: caller LLRs of `elem` bytes each (4: fp32, 2: bf16).
 static int decode_host(ldpc_handle* h, const ldpc_run_params* p, const void* llr, int elem, int64_t n, float* post,
                        int32_t* iters, int32_t* synd_fail, int32_t* bit_errors, ldpc_tally* out) {
@@ -1026,6 +1137,17 @@ static int decode_host(ldpc_handle* h, const ldpc_run_params* p, const void* llr
     CU(cudaSetDevice(h->device));
     const size_t ntx = (size_t)(h->N - h->P);
     const size_t nb = (size_t)n;
+    ldpc_run_params q = *p;
+    q.first_frame = 0;
+    q.n_frames = nb;
+    // A page-locked array is copied by DMA straight from the caller's memory; a pageable one through
+    // the handle's pinned ring, filled by host threads.
+    bool pageable = true;
+    const bool plain = !nb || (host_memory(llr, &pageable) && (!post || host_memory(post)) && (!iters || host_memory(iters)) &&
+                               (!synd_fail || host_memory(synd_fail)) && (!bit_errors || host_memory(bit_errors)));
+    if (nb && plain && nb <= ldpc_handle::kSmallBytes && nb * ntx * sizeof(float) <= ldpc_handle::kSmallBytes &&
+        3 * nb * sizeof(int32_t) + (post ? nb * h->N * sizeof(float) : 0) <= ldpc_handle::kSmallBytes)
+        return decode_small(h, &q, llr, elem, nb, post, iters, synd_fail, bit_errors, out);
     if (nb) {
         if ((rc = ensure_cap((void**)&h->d_llr, &h->llr_cap, nb * ntx * sizeof(float)))) return rc;
         if (elem == 2 && (rc = ensure_cap((void**)&h->d_llr16, &h->llr16_cap, nb * ntx * sizeof(uint16_t))))
@@ -1037,25 +1159,12 @@ static int decode_host(ldpc_handle* h, const ldpc_run_params* p, const void* llr
         return fail(LDPC_EIO, "copy stream creation failed");
     if (!h->cev && cudaEventCreateWithFlags(&h->cev, cudaEventDisableTiming) != cudaSuccess)
         return fail(LDPC_EIO, "copy event creation failed");
-    // A page-locked array is copied by DMA straight from the caller's memory; a pageable one through
-    // the handle's pinned ring, filled by host threads.
-    bool pageable = true;
-    if (nb) {
-        cudaPointerAttributes a;
-        if (cudaPointerGetAttributes(&a, llr) == cudaSuccess)
-            pageable = a.type == cudaMemoryTypeUnregistered;
-        else
-            cudaGetLastError();
-    }
     // Large calls copy the LLRs in chunks on the copy stream, so that the decoding of one chunk
     // overlaps the copy of the next; small ones are one chunk.
     constexpr uint64_t kMinChunk = 8192;
     uint64_t chunk = kMaxLaunchFrames;
     if (nb >= 2 * kMinChunk) chunk = std::min<uint64_t>(kMaxLaunchFrames, std::max<uint64_t>(kMinChunk, (nb + 7) / 8));
     const HostLlr hin{llr, elem, pageable};
-    ldpc_run_params q = *p;
-    q.first_frame = 0;
-    q.n_frames = nb;
     int32_t* d_it = h->d_frame_out;
     int32_t* d_sf = d_it ? d_it + nb : nullptr;
     int32_t* d_be = d_sf ? d_sf + nb : nullptr;
@@ -1063,7 +1172,25 @@ static int decode_host(ldpc_handle* h, const ldpc_run_params* p, const void* llr
                          nb ? &hin : nullptr, chunk)))
         return rc;
     if (nb) {
-        if (post) CU(cudaMemcpyAsync(post, h->d_post, nb * h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        bool ring = false;
+        if (post && host_memory(post, &ring) && ring) {
+            if ((rc = unstage_d2h(h, reinterpret_cast<char*>(post), reinterpret_cast<const char*>(h->d_post),
+                                  nb * h->N * sizeof(float))))
+                return rc;
+        } else if (post) {
+            CU(cudaMemcpyAsync(post, h->d_post, nb * h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        }
+        // the per-frame counts: one copy into the pinned buffer where they fit, else one per array
+        if (plain && 3 * nb * sizeof(int32_t) <= ldpc_handle::kSmallBytes) {
+            if ((rc = small_alloc(h))) return rc;
+            CU(cudaMemcpyAsync(h->h_small, d_it, 3 * nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+            if ((rc = read_tally(h, out))) return rc;
+            const int32_t* o = reinterpret_cast<const int32_t*>(h->h_small);
+            if (iters) memcpy(iters, o, nb * sizeof(int32_t));
+            if (synd_fail) memcpy(synd_fail, o + nb, nb * sizeof(int32_t));
+            if (bit_errors) memcpy(bit_errors, o + 2 * nb, nb * sizeof(int32_t));
+            return 0;
+        }
         if (iters) CU(cudaMemcpyAsync(iters, d_it, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
         if (synd_fail) CU(cudaMemcpyAsync(synd_fail, d_sf, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
         if (bit_errors) CU(cudaMemcpyAsync(bit_errors, d_be, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
@@ -1175,7 +1302,7 @@ extern "C" int ldpc_snr_bins(ldpc_handle* h, uint64_t* out) {
 }
 
 // ----------------------------------------------------------------------------- batched launch
-// Several codes decoded by one CUDA graph launch: per code, memset nodes for its counters followed by
+// Several codes decoded by one CUDA graph launch: per code, a memset node for its counters followed by
 // its persistent kernel; the codes' kernels have no dependencies on one another and run side by
 // side, each on its share of the GPU's CTA slots, each claiming frames from its own queue.  The graph
 // is built and instantiated once and relaunched: a call updates its kernel nodes in place
@@ -1330,14 +1457,10 @@ extern "C" int ldpc_batch_run(ldpc_batch* b, const ldpc_run_params* params, cons
         cudaGraphNode_t chain = nullptr;  // the last chained kernel node
         for (int i = 0; i < n && !rc; ++i) {
             ldpc_handle* h = b->hs[i];
-            cudaGraphNode_t deps[5];
-            if ((rc = add_memset(g, h->d_tally, TALLY_WORDS * sizeof(unsigned long long), &deps[0])) ||
-                (rc = add_memset(g, h->d_work, 64, &deps[1])) ||
-                (rc = add_memset(g, h->d_hist, h->hist_bins * sizeof(unsigned long long), &deps[2])) ||
-                (rc = add_memset(g, h->d_snr, 4 * SNR_BINS * sizeof(unsigned long long), &deps[3])))
-                break;
+            cudaGraphNode_t deps[2];
+            if ((rc = add_memset(g, h->d_io, ldpc_handle::kCounterBytes, &deps[0]))) break;
             if (!key[i]) continue;
-            int nd = 4;
+            int nd = 1;
             if (key[i] == 2 && chain) deps[nd++] = chain;
             void* args[] = {&Ls[i].qp};
             const cudaKernelNodeParams kp = kparams(i, args);

@@ -99,15 +99,23 @@ static const QcEntry qc_r12k1[] = {
     // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
     LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 6, 5),
     LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 5, 5),
+    // layout 6 with more registers, for calls of few frames
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_BF16, ALGO_AMIN, false, false, 5, 5),
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP16, ALGO_AMIN, false, false, 5, 5),
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_BF16, ALGO_AMIN, false, true, 5, 5),
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP16, ALGO_AMIN, false, true, 5, 5),
+    LDPC_QC_ENTRY_RF(128, 6, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 0, 5),
 };
 LDPC_QC_REGISTER(qc_r12k1)
 
 // Default shapes (us of the kernel at 1 / 440 / 1500 / 100000 frames, 2.04 dB, Approximate-Min*).  Below about
-// 1500 frames a kernel waits for its slowest frame and fewer registers per thread do not help; above,
-// resident warps and instructions decide.
-//   bf16: cap 5 25.0 / 47.5 / 110.8 / 5831, layout 6 cap 8 27.6 / 50.2 / 108.6 / 5269, layout 2 cap 8 - / 53.5 / 109.0 / 5335,
+// 2500 frames a kernel waits for its slowest frame and fewer registers per thread do not help; above,
+// resident warps and instructions decide.  (Layout 6 cap 5 at 1 / 440 / 1500 frames, 2.0 dB, all other kernels timed
+// again beside it: bf16 21.5 / 48.1 / 105.5, cap 8 25.6 / 54.1 / 109.5, layout 0 cap 5 22.5 / 50.2 / 113.6; fp16 20.5 / 48.2 /
+// 102.4, layout 0 cap 5 21.5 / 52.2 / 117.8.)
+//   bf16: layout 0 cap 5 25.0 / 47.5 / 110.8 / 5831, layout 6 cap 8 27.6 / 50.2 / 108.6 / 5269, layout 2 cap 8 - / 53.5 / 109.0 / 5335,
 //         (1,1,0,0) 26.9 / 52.2 / 119.0 / 6268
-//   fp16: cap 5 23.5 / 46.3 / 110.8 / 5780, layout 2 cap 6 26.8 / 47.5 / 104.9 / 5171, layout 6 cap 6 24.9 / 45.4 / 104.8 /
+//   fp16: layout 0 cap 5 23.5 / 46.3 / 110.8 / 5780, layout 2 cap 6 26.8 / 47.5 / 104.9 / 5171, layout 6 cap 6 24.9 / 45.4 / 104.8 /
 //         5218, (1,1,0,0) 24.9 / 49.2 / 114.0 / 5966
 //   fp32: layout 6 21.0 / 39.3 / 95.6 / 5057, its cap 5 22.8 / 39.1 / 92.5 / 4664, layout 2 cap 5 26.8 / 45.4 / 94.7 / 4678,
 //         (1,1,0,0) 22.8 / 43.3 / 96.4 / 5143
@@ -118,10 +126,14 @@ static const QcDefault qc_r12k1_default[] = {
     {128, 6, STORE_FP32, ALGO_WAMIN, 1500, 1, 1, 0, 2},
     {128, 6, STORE_FP32, ALGO_WAMIN, 0, 1, 1, 0, 0},
     {128, 6, STORE_FP16, ALGO_WAMIN, 0, 1, 1, 5, 0},
+    {128, 6, STORE_BF16, -1, 2500, 1, 1, 8, 6},
+    {128, 6, STORE_BF16, -1, 0, 1, 1, 5, 6},
     {128, 6, STORE_BF16, -1, 1500, 1, 1, 8, 6},
     {128, 6, STORE_BF16, -1, 1500, 1, 1, 8, 2},
     {128, 6, STORE_BF16, -1, 1500, 1, 1, 0, 2},
     {128, 6, STORE_BF16, -1, 0, 1, 1, 5, 0},
+    {128, 6, STORE_FP16, -1, 2500, 1, 1, 6, 2},
+    {128, 6, STORE_FP16, -1, 0, 1, 1, 5, 6},
     {128, 6, STORE_FP16, -1, 1500, 1, 1, 6, 2},
     {128, 6, STORE_FP16, -1, 1500, 1, 1, 6, 6},
     {128, 6, STORE_FP16, -1, 1500, 1, 1, 0, 2},

@@ -101,10 +101,9 @@ def load(path: str = LIB_PATH):
     L.ldpc_destroy.restype = None
     L.ldpc_kernel_kind.argtypes = [C.c_void_p]
     L.ldpc_run_chunk.argtypes = [C.c_void_p, P(RunParams), P(Tally)]
-    L.ldpc_decode_llr.argtypes = [C.c_void_p, P(RunParams), P(C.c_float), C.c_int64, P(C.c_float),
-                                  P(C.c_int32), P(C.c_int32), P(C.c_int32), P(Tally)]
-    L.ldpc_decode_llr_bf16.argtypes = [C.c_void_p, P(RunParams), P(C.c_uint16), C.c_int64, P(C.c_float),
-                                       P(C.c_int32), P(C.c_int32), P(C.c_int32), P(Tally)]
+    # the arrays as plain addresses: a typed pointer object costs microseconds per argument
+    L.ldpc_decode_llr.argtypes = [C.c_void_p, P(RunParams), C.c_void_p, C.c_int64] + [C.c_void_p] * 4 + [P(Tally)]
+    L.ldpc_decode_llr_bf16.argtypes = L.ldpc_decode_llr.argtypes
     L.ldpc_channel_llr.argtypes = [C.c_void_p, P(RunParams), P(C.c_float)]
     L.ldpc_iter_histogram.argtypes = [C.c_void_p, P(C.c_uint64), C.c_int]
     L.ldpc_snr_bins.argtypes = [C.c_void_p, P(C.c_uint64)]
@@ -362,12 +361,9 @@ class Decoder:
         sf = np.empty(n, np.int32)
         be = np.empty(n, np.int32)
         t = Tally()
-        if bf16:
-            _check(self._lib.ldpc_decode_llr_bf16(self._h, C.byref(p), llr.ctypes.data_as(C.POINTER(C.c_uint16)),
-                                                  n, _fp(post), _ip(it), _ip(sf), _ip(be), C.byref(t)))
-        else:
-            _check(self._lib.ldpc_decode_llr(self._h, C.byref(p), _fp(llr), n, _fp(post), _ip(it), _ip(sf),
-                                             _ip(be), C.byref(t)))
+        f = self._lib.ldpc_decode_llr_bf16 if bf16 else self._lib.ldpc_decode_llr
+        _check(f(self._h, C.byref(p), llr.ctypes.data, n, post.ctypes.data if want_post else None, it.ctypes.data,
+                 sf.ctypes.data, be.ctypes.data, C.byref(t)))
         return post, it, sf, be, ChunkResult(t.frames, t.bit_errors, t.frame_errors, t.iter_sum,
                                              t.unconverged, t.max_iters, t.kernel_ms, t.bit_errors_sq)
 
