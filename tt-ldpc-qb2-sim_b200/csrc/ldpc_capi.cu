@@ -58,11 +58,22 @@ void register_qc_defaults(QcDefaults* t) {
 const QcDefaults* qc_defaults() { return g_defaults; }
 }  // namespace ldpcb200
 
-static const void* find_qc(const QcKey& k) {
+// scaled: whether an entry that decodes at LLR_SCALE will do.
+static const QcEntry* find_qc(const QcKey& k, bool scaled) {
     for (const QcTable* t = qc_tables(); t; t = t->next)
         for (int i = 0; i < t->count; ++i)
-            if (t->entries[i].key == k) return t->entries[i].fn;
+            if (t->entries[i].key == k && (scaled || !t->entries[i].scaled)) return &t->entries[i];
     return nullptr;
+}
+
+// Whether the scaled kernels may decode a simulated channel: LLR mean and deviation between 2^-10 and 2^12 (or 0),
+// i.e. an Eb/N0 between about -30 and 30 dB, and at most 10000 iterations; values then stay far inside the
+// range LLR_SCALE leaves, and the kernel checks long frames all the same.
+static bool qc_scaled_ok(const ldpc_run_params* p) {
+    auto in = [](float v) { return v == 0.0f || (v >= 9.765625e-4f && v <= 4096.0f); };
+    const bool snr = p->ebn0_hi_db > p->ebn0_lo_db;
+    return p->max_iter <= 10000 &&
+           (snr ? p->ebn0_lo_db >= -30.0f && p->ebn0_hi_db <= 30.0f : in(p->mu < 0.0f ? -p->mu : p->mu) && in(p->sigma));
 }
 
 // ----------------------------------------------------------------------------- handle
@@ -366,9 +377,10 @@ extern "C" int64_t ldpc_launch_param_bytes(const ldpc_handle* h) {
     return h->kind == LDPC_KERNEL_QC ? (int64_t)sizeof(QcParams) : (int64_t)sizeof(GenParams);
 }
 
-static const void* find_shape(const ldpc_handle* h, int storage, int algo, int clip, int ext, int R, int F, int B, int G) {
+static const QcEntry* find_shape(const ldpc_handle* h, int storage, int algo, int clip, int ext, int R, int F, int B,
+                                 int G, bool scaled = true) {
     if ((G == 5 || G == 6) && h->fix < 0) return nullptr;  // compiled-in descriptors of another code
-    return find_qc(QcKey{h->Z, h->D, R, F, storage, algo, clip, ext, B, G});
+    return find_qc(QcKey{h->Z, h->D, R, F, storage, algo, clip, ext, B, G}, scaled);
 }
 
 // The default shape of a numerics variant for a call of n frames: the first line of the defaults that
@@ -376,10 +388,12 @@ static const void* find_shape(const ldpc_handle* h, int storage, int algo, int c
 // built, else the first shape built for it (e.g. the global-message kernel of a K = 16384 code).
 // scratch = false leaves out the lines that need a message scratch.
 namespace ldpcb200 {
-const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4]) {
+const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4],
+                       bool scaled) {
     auto built = [&](int R, int F, int B, int G) -> const void* {
         if ((G == 5 || G == 6) && fix < 0) return nullptr;  // compiled-in descriptors of another code
-        return find_qc(QcKey{Z, D, R, F, storage, algo, clip, ext, B, G});
+        const QcEntry* e = find_qc(QcKey{Z, D, R, F, storage, algo, clip, ext, B, G}, scaled);
+        return e ? e->fn : nullptr;
     };
     for (int own = 1; own >= 0; --own)
         for (const QcDefaults* t = qc_defaults(); t; t = t->next)
@@ -401,7 +415,7 @@ const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, i
         for (int i = 0; i < t->count; ++i) {
             const QcKey& k = t->entries[i].key;
             if (k.Z == Z && k.D == D && k.mode == storage && k.algo == algo && k.clip == clip && k.ext == ext &&
-                ((k.G != 5 && k.G != 6) || fix >= 0)) {
+                ((k.G != 5 && k.G != 6) || fix >= 0) && (scaled || !t->entries[i].scaled)) {
                 s[0] = k.R; s[1] = k.F; s[2] = k.B; s[3] = k.G;
                 return t->entries[i].fn;
             }
@@ -411,13 +425,13 @@ const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, i
 }  // namespace ldpcb200
 
 static bool default_shape(const ldpc_handle* h, int storage, int algo, int clip, int ext, uint32_t n, bool scratch,
-                          int s[4]) {
-    return qc_default(h->Z, h->D, h->fix, storage, algo, clip, ext, n, scratch, s) != nullptr;
+                          bool scaled, int s[4]) {
+    return qc_default(h->Z, h->D, h->fix, storage, algo, clip, ext, n, scratch, s, scaled) != nullptr;
 }
 
 static bool default_shape_exists(const ldpc_handle* h, int storage, int algo) {
     int s[4];
-    return default_shape(h, storage, algo, 0, 0, 0, true, s);
+    return default_shape(h, storage, algo, 0, 0, 0, true, true, s);
 }
 
 extern "C" int ldpc_set_weights(ldpc_handle* h, const float* alpha, const float* beta, int n_iter, int n_classes,
@@ -639,7 +653,7 @@ struct QcLaunch {
 
 static double code_rate(const ldpc_handle* h) { return (double)(h->N - h->M) / (double)(h->N - h->P); }
 
-static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void* fn, const int* sh, bool wrow, bool ext,
+static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const QcEntry* entry, const int* sh, bool wrow, bool ext,
                             uint32_t n, uint64_t first, const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf,
                             int32_t* d_be, double grid_frac, QcLaunch* out);
 
@@ -647,30 +661,32 @@ static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void
 // launch that share of the GPU's resident CTA slots (for kernels that run side by side).
 static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32_t n, uint64_t first,
                       const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be,
-                      double grid_frac, QcLaunch* out) {
+                      double grid_frac, QcLaunch* out, bool scaled) {
+    scaled = scaled && !ext && qc_scaled_ok(p);
     const bool clip = p->l_max > 0.0f || p->r_max > 0.0f || p->l_post_max > 0.0f;
     int sh[4];
     bool chosen = false, scratch = true;
     // the handle's shape for this storage, else the default shape of the algorithm
-    auto lookup = [&](int algo) -> const void* {
+    auto lookup = [&](int algo) -> const QcEntry* {
         int s[4] = {h->shape[p->storage][0], h->shape[p->storage][1], h->shape[p->storage][2],
                     h->shape[p->storage][3]};
-        const void* f = nullptr;
+        const QcEntry* f = nullptr;
         if (s[0] || s[1] || s[2] || s[3])
-            f = find_shape(h, p->storage, algo, clip, ext, s[0] ? s[0] : 1, s[1] ? s[1] : 1, s[2], s[3]);
+            f = find_shape(h, p->storage, algo, clip, ext, s[0] ? s[0] : 1, s[1] ? s[1] : 1, s[2], s[3],
+                           scaled);
         chosen = f != nullptr;
         if (f) {
             s[0] = s[0] ? s[0] : 1;
             s[1] = s[1] ? s[1] : 1;
-        } else if (default_shape(h, p->storage, algo, clip, ext, n, scratch, s)) {
-            f = find_shape(h, p->storage, algo, clip, ext, s[0], s[1], s[2], s[3]);
+        } else if (default_shape(h, p->storage, algo, clip, ext, n, scratch, scaled, s)) {
+            f = find_shape(h, p->storage, algo, clip, ext, s[0], s[1], s[2], s[3], scaled);
         }
         if (f) std::copy(s, s + 4, sh);
         return f;
     };
     // weights with one class per row run on the per-row weighted kernels where they are built
     const bool wrow = p->algo == LDPC_ALGO_WAMIN && h->w_row && lookup(ALGO_WROW);
-    const void* fn = lookup(wrow ? ALGO_WROW : p->algo);
+    const QcEntry* fn = lookup(wrow ? ALGO_WROW : p->algo);
     if (!fn) return LDPC_ENOTSUP;  // the caller falls back to the general kernel
     int rc = prepare_qc_shape(h, p, fn, sh, wrow, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, grid_frac, out);
     if (rc == LDPC_ENOMEM && !chosen && qc_shape_in_scratch(sh[3])) {
@@ -683,10 +699,11 @@ static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32
     return rc;
 }
 
-static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void* fn, const int* sh, bool wrow, bool ext,
+static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const QcEntry* entry, const int* sh, bool wrow, bool ext,
                             uint32_t n, uint64_t first, const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf,
                             int32_t* d_be, double grid_frac, QcLaunch* out) {
     const int R = sh[0], F = sh[1], G = sh[3];
+    const void* fn = entry->fn;
     QcParams& qp = out->qp;
     memset(&qp, 0, sizeof qp);
     memcpy(qp.blk_off, h->blk_off, sizeof qp.blk_off);
@@ -742,9 +759,10 @@ static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void
             memcpy(&v, &u, 4);
             return v;
         };
-        qp.circ_c[0] = c(0.69315f);
+        const float scale = entry->scaled ? LLR_SCALE : 1.0f;
+        qp.circ_c[0] = c(0.69315f) * scale;
         qp.circ_c[1] = c(-0.40f);
-        qp.circ_c[2] = c(0.65715f);
+        qp.circ_c[2] = c(0.65715f) * scale;
         qp.circ_c[3] = c(-0.328f);
         qp.circ_damping = h->circ.damping;
         qp.circ_sfpu = sfpu ? 1 : 0;
@@ -778,9 +796,9 @@ static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const void
 }
 
 static int launch_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32_t n, uint64_t first,
-                     const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be) {
+                     const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be, bool scaled) {
     QcLaunch L;
-    int rc = prepare_qc(h, p, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, 1.0, &L);
+    int rc = prepare_qc(h, p, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, 1.0, &L, scaled);
     if (rc || L.grid == 0) return rc;
     void* args[] = {&L.qp};
     CU(cudaLaunchKernel(L.fn, dim3(L.grid), dim3(L.block), args, L.smem, h->stream));
@@ -964,7 +982,7 @@ static int stage_h2d(ldpc_handle* h, void* dst, const char* src, size_t bytes) {
 // previous chunk decodes; chunk <= kMaxLaunchFrames.
 static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64_t n, const float* d_llr,
                       float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be, const HostLlr* hin = nullptr,
-                      uint64_t chunk = kMaxLaunchFrames) {
+                      uint64_t chunk = kMaxLaunchFrames, bool scaled = true) {
     int rc;
     if ((rc = reset_counters(h))) return rc;
     if (n == 0) CU(cudaEventRecord(h->ev0, h->stream));
@@ -998,7 +1016,7 @@ static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64
         int32_t* sf = d_sf ? d_sf + off : nullptr;
         int32_t* be = d_be ? d_be + off : nullptr;
         rc = LDPC_ENOTSUP;
-        if (h->kind == LDPC_KERNEL_QC) rc = launch_qc(h, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be);
+        if (h->kind == LDPC_KERNEL_QC) rc = launch_qc(h, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be, scaled);
         if (rc == LDPC_ENOTSUP && p->algo == LDPC_ALGO_WAMIN)
             return fail(LDPC_ENOTSUP, "the weighted decoder is not built for Z=%d D=%d with storage %d", h->Z, h->D,
                         p->storage);
@@ -1017,7 +1035,7 @@ static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64
             if (sh[3] != GEN_LAYOUT_WARP)
                 rc = launch_general_step(&h->gen, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be,
                                          h->d_tally, h->d_hist, h->hist_bins, h->d_work, h->n_sm, h->stream, g_err,
-                                         h->d_snr);
+                                         h->d_snr, scaled && qc_scaled_ok(p));
             if (rc == LDPC_ENOTSUP)
                 rc = launch_general(&h->gen, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be, h->d_tally,
                                     h->d_hist, h->hist_bins, h->d_work, h->n_sm, h->stream, g_err, h->d_snr);
@@ -1035,6 +1053,12 @@ extern "C" int ldpc_run_chunk(ldpc_handle* h, const ldpc_run_params* p, ldpc_tal
     if ((rc = check_params(h, p))) return rc;
     CU(cudaSetDevice(h->device));
     if ((rc = run_frames(h, p, false, p->n_frames, nullptr, nullptr, nullptr, nullptr, nullptr))) return rc;
+    if ((rc = read_tally(h, out))) return rc;
+    if (!h->h_tally[T_OUT_OF_RANGE]) return 0;
+    // a frame's values left the scaled kernels' range: the same frames on the unscaled ones
+    if ((rc = run_frames(h, p, false, p->n_frames, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, kMaxLaunchFrames,
+                         false)))
+        return rc;
     return read_tally(h, out);
 }
 
@@ -1382,8 +1406,19 @@ static int add_memset(cudaGraph_t g, void* dst, size_t bytes, cudaGraphNode_t* n
     return 0;
 }
 
+static int batch_run(ldpc_batch* b, const ldpc_run_params* params, const float* share, ldpc_tally* out, float* graph_ms,
+                     bool scaled, bool* out_of_range);
+
 extern "C" int ldpc_batch_run(ldpc_batch* b, const ldpc_run_params* params, const float* share, ldpc_tally* out,
                               float* graph_ms) {
+    bool far = false;
+    const int rc = batch_run(b, params, share, out, graph_ms, true, &far);
+    // a frame's values left the scaled kernels' range: the same frames on the unscaled ones
+    return rc || !far ? rc : batch_run(b, params, share, out, graph_ms, false, &far);
+}
+
+static int batch_run(ldpc_batch* b, const ldpc_run_params* params, const float* share, ldpc_tally* out, float* graph_ms,
+                     bool scaled, bool* out_of_range) {
     if (!b || !params) return fail(LDPC_EINVAL, "bad arguments");
     CU(cudaSetDevice(b->device));
     const int n = (int)b->hs.size();
@@ -1409,7 +1444,7 @@ extern "C" int ldpc_batch_run(ldpc_batch* b, const ldpc_run_params* params, cons
         // next code's CTAs as the previous code's retire
         const double frac = (share && work_total > 0.0) ? w[i] / work_total : 1.0;
         rc = prepare_qc(b->hs[i], &params[i], false, (uint32_t)params[i].n_frames, params[i].first_frame, nullptr,
-                        nullptr, nullptr, nullptr, nullptr, frac, &Ls[i]);
+                        nullptr, nullptr, nullptr, nullptr, frac, &Ls[i], scaled);
         if (rc == LDPC_ENOTSUP) return fail(LDPC_ENOTSUP, "code %d: no QC kernel for these options", i);
         if (rc) return rc;
         if (!Ls[i].grid) continue;
@@ -1497,6 +1532,7 @@ extern "C" int ldpc_batch_run(ldpc_batch* b, const ldpc_run_params* params, cons
         h->launches += params[i].n_frames ? 1 : 0;
         unsigned long long t[TALLY_WORDS];
         CU(cudaMemcpy(t, h->d_tally, sizeof t, cudaMemcpyDeviceToHost));
+        *out_of_range |= t[T_OUT_OF_RANGE] != 0;
         if (out) {
             out[i].frames = t[T_FRAMES];
             out[i].bit_errors = t[T_BIT_ERR];

@@ -91,7 +91,7 @@ int build_general_steps(const int32_t* rows, int dmax, GeneralCode* g, std::stri
 int launch_general_step(GeneralCode* g, const ldpc_run_params* p, bool ext, uint32_t n, uint64_t first,
                         const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be,
                         unsigned long long* d_tally, unsigned long long* d_hist, int hist_bins, unsigned int* d_work,
-                        int n_sm, cudaStream_t stream, std::string& err, unsigned long long* d_snr_bins);
+                        int n_sm, cudaStream_t stream, std::string& err, unsigned long long* d_snr_bins, bool scaled);
 int launch_general(GeneralCode* g, const ldpc_run_params* p, bool ext, uint32_t n, uint64_t first,
                    const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be,
                    unsigned long long* d_tally, unsigned long long* d_hist, int hist_bins, unsigned int* d_work,

@@ -88,7 +88,8 @@ struct QcStructure {
     int32_t blk_off[QC_LAYERS][QC_DMAX], shift[QC_LAYERS][QC_DMAX];
 };
 bool qc_structure(const int32_t* rows, int N, int M, int P, int dmax, QcStructure* out);
-const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4]);
+const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4],
+                       bool scaled = false);
 void qc_message_layout(QcParams* qp, int Z, int D);
 size_t qc_smem_bytes(int N, int Z, int D, int R, int F, int G, int storage);
 
@@ -100,7 +101,9 @@ __host__ __device__ constexpr int qc_edge_slot(int l, int e, int D) {
 }
 
 enum TallyWord : int {
-    T_FRAMES = 0, T_BIT_ERR, T_FRAME_ERR, T_ITER_SUM, T_UNCONVERGED, T_MAX_ITER, T_BIT_ERR_SQ, TALLY_WORDS = 8
+    T_FRAMES = 0, T_BIT_ERR, T_FRAME_ERR, T_ITER_SUM, T_UNCONVERGED, T_MAX_ITER, T_BIT_ERR_SQ,
+    T_OUT_OF_RANGE,  // set by a scaled kernel whose values left its range (LLR_SCALE)
+    TALLY_WORDS = 8
 };
 
 template <int MODE> struct LTraits;
@@ -237,12 +240,14 @@ __device__ __forceinline__ RowMsgGlobal<d, MODE> rg_row(const QcParams& p, size_
 // other operand unchanged, so only a row with fewer than two real edges needs care: its chain over
 // the other edges then holds no real value (above 1e38), and the reference's m_others is the row's
 // minimum (ldpc_decoder_core.h:180-181).
-template <int d, int MODE, int ALGO, bool CLIP, int F, class MSG, bool BO = false, bool PAD = false>
+// SC: posteriors, messages and magnitudes are scaled by LLR_SCALE (amin_step_scaled).
+template <int d, int MODE, int ALGO, bool CLIP, int F, class MSG, bool BO = false, bool PAD = false, bool SC = false>
 __device__ __forceinline__ void row_update(const int (&idx)[d], typename LTraits<MODE>::T* sL, int lstride,
                                            MSG (&rm)[F], float r_cap, float lp_cap,
                                            const float2* const* wt = nullptr) {
     using LT = LTraits<MODE>;
     using LE = typename LT::T;
+    constexpr float AM_INIT = SC ? 9999.0f * LLR_SCALE : 9999.0f;
     auto lptr = [&](int f, int e) -> LE* {
         if constexpr (BO) return reinterpret_cast<LE*>(reinterpret_cast<char*>(sL + f * lstride) + idx[e]);
         else return sL + f * lstride + idx[e];
@@ -281,7 +286,7 @@ __device__ __forceinline__ void row_update(const int (&idx)[d], typename LTraits
                 // predicate registers and were packed into and tested out of general registers:
                 // +4-5 % on the rate-4/5 kernels, fewer spills at 64 registers; at degree 10 the
                 // prefix form stays faster (r2/3 K=1024 26.0 against 25.2 M frames/s).
-                float m1 = 9999.0f;
+                float m1 = AM_INIT;
                 int am = 0;
 #pragma unroll
                 for (int e = 0; e < d; ++e) {
@@ -293,7 +298,7 @@ __device__ __forceinline__ void row_update(const int (&idx)[d], typename LTraits
                 for (int i = 0; i < d; ++i) lt[i] = (i + 1 < d) ? (i < am) : false;
             } else {
                 float pm[d];
-                pm[0] = fminf(a[0], 9999.0f);
+                pm[0] = fminf(a[0], AM_INIT);
 #pragma unroll
                 for (int e = 1; e < d; ++e) pm[e] = fminf(pm[e - 1], a[e]);
                 mn = pm[d - 1];
@@ -304,10 +309,14 @@ __device__ __forceinline__ void row_update(const int (&idx)[d], typename LTraits
             for (int e = 0; e < d; ++e) is_am[e] = (e == 0 ? true : lt[e - 1]) && !lt[e];
             float m = fabsf(lt[0] ? q[f][0] : q[f][1]);
 #pragma unroll
-            for (int i = 1; i + 1 < d; ++i) m = amin_step_fma(m, fabsf(lt[i] ? q[f][i] : q[f][i + 1]));
-            if (PAD) m = m > 1e38f ? mn : m;
+            for (int i = 1; i + 1 < d; ++i) {
+                const float o = fabsf(lt[i] ? q[f][i] : q[f][i + 1]);
+                m = SC ? amin_step_scaled(m, o) : amin_step_fma(m, o);
+            }
+            // (scaled, a chain of padded edges only has saturated at 1)
+            if (PAD) m = m > (SC ? 0.5f : 1e38f) ? mn : m;
             mag_min = m;
-            mag_all = amin_step_fma(m, mn);
+            mag_all = SC ? amin_step_scaled(m, mn) : amin_step_fma(m, mn);
         } else {
             // normalised min-sum, alpha = 0.75 (ldpc_decoder_core.h:322-379)
             int am = 0;
@@ -378,7 +387,7 @@ struct CircRt {
     float damping;
     bool sfpu;
 };
-template <int d, int MODE, int F, class MSG, bool BO = false>
+template <int d, int MODE, int F, class MSG, bool BO = false, bool SC = false>
 __device__ __forceinline__ void row_update_circ(const int (&idx)[d], typename LTraits<MODE>::T* sL, int lstride,
                                                 MSG (&rm)[F], const CircRt& cr) {
     static_assert(d == 3 || d == 6, "the circulant engine's rows have degree 3 or 6");
@@ -401,18 +410,18 @@ __device__ __forceinline__ void row_update_circ(const int (&idx)[d], typename LT
         }
         par &= 0x80000000u;
         if constexpr (d == 6) {
-            const float m03 = circ_g(a[0], a[3], cr.k), m14 = circ_g(a[1], a[4], cr.k), m25 = circ_g(a[2], a[5], cr.k);
-            const float o0 = circ_g(m14, m25, cr.k), o1 = circ_g(m03, m25, cr.k), o2 = circ_g(m03, m14, cr.k);
-            mag[0] = circ_g(o0, a[3], cr.k);
-            mag[3] = circ_g(o0, a[0], cr.k);
-            mag[1] = circ_g(o1, a[4], cr.k);
-            mag[4] = circ_g(o1, a[1], cr.k);
-            mag[2] = circ_g(o2, a[5], cr.k);
-            mag[5] = circ_g(o2, a[2], cr.k);
+            const float m03 = circ_g<SC>(a[0], a[3], cr.k), m14 = circ_g<SC>(a[1], a[4], cr.k), m25 = circ_g<SC>(a[2], a[5], cr.k);
+            const float o0 = circ_g<SC>(m14, m25, cr.k), o1 = circ_g<SC>(m03, m25, cr.k), o2 = circ_g<SC>(m03, m14, cr.k);
+            mag[0] = circ_g<SC>(o0, a[3], cr.k);
+            mag[3] = circ_g<SC>(o0, a[0], cr.k);
+            mag[1] = circ_g<SC>(o1, a[4], cr.k);
+            mag[4] = circ_g<SC>(o1, a[1], cr.k);
+            mag[2] = circ_g<SC>(o2, a[5], cr.k);
+            mag[5] = circ_g<SC>(o2, a[2], cr.k);
         } else {
-            mag[0] = circ_g(a[1], a[2], cr.k);
-            mag[1] = circ_g(a[0], a[2], cr.k);
-            mag[2] = circ_g(a[0], a[1], cr.k);
+            mag[0] = circ_g<SC>(a[1], a[2], cr.k);
+            mag[1] = circ_g<SC>(a[0], a[2], cr.k);
+            mag[2] = circ_g<SC>(a[0], a[1], cr.k);
         }
         float rn[d];
 #pragma unroll
@@ -643,12 +652,14 @@ __device__ __forceinline__ int qc_shift(const QcParams& p, int l, int e) {
 // words (T * (12 + 8 D) words); one row per thread.
 // FIX: >= 0 for the descriptors of a known code compiled in (layouts 5 and 6; the host offers them
 // only for a matrix whose descriptors are those).
+// SC: the frames are decoded at LLR_SCALE (the simulation of Approximate-Min* or the circulant engine's decoder,
+// fp32 or bf16 storage, no clips): the same tallies, one instruction less per min* step.
 // ROLL (layout 7, global messages only): the eight degree-D layers run as one loop that is not
 // unrolled, each row's descriptors read from the kernel parameters by layer index.  The unrolled
 // body of a degree-18 code is tens of KB of instructions; with one-warp CTAs whose warps are
 // each at a different point of it, the instruction fetch stalls the SM.
 template <int Z, int D, int R, int F, int MODE, int ALGO, bool CLIP, bool EXT, int B = 0, bool PAIR = false,
-          bool RG = false, bool OT = false, int FIX = -1, bool ROLL = false>
+          bool RG = false, bool OT = false, int FIX = -1, bool ROLL = false, bool SC = false>
 __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_constant__ QcParams p) {
     constexpr int T = Z / R;
     constexpr int W = Z / 32;  // 32-bit words per Z-bit block vector
@@ -660,6 +671,8 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
     static_assert(!OT || (!PAIR && !RG && R == 1), "the offset table is built for one row per thread");
     static_assert(FIX < 0 || (!OT && !PAIR && FIX < QC_FIXED_COUNT), "compiled-in descriptors: no offset table");
     constexpr bool CIRC = ALGO == ALGO_CIRC;
+    static_assert(!SC || (!EXT && !CLIP && !PAIR && MODE != STORE_FP16 && (CIRC || ALGO == ALGO_AMIN)),
+                  "scaled decoding: the simulation, no clips, no fp16 messages");
     static_assert(!ROLL || (RG && FIX < 0 && !CIRC), "the rolled layer loop: global messages, parameter descriptors");
     static_assert(!CIRC || (D == 6 && !CLIP && !PAIR), "the circulant engine's decoder: degrees 3 and 6, no clips");
     using SV = SlotView<MODE, PAIR>;
@@ -760,6 +773,10 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                     if (per_frame_snr)
                         frame_snr(p.ebn0_lo, p.ebn0_hi, p.rate, gf, p.stream, p.seed_lo, p.seed_hi, ch_mu, ch_sigma,
                                   snr_bin[f]);
+                    if (SC) {
+                        ch_mu *= LLR_SCALE;
+                        ch_sigma *= LLR_SCALE;
+                    }
                     for (int qd = tid; qd < nq; qd += T) {
                         float n[4];
                         if (ch_sigma > 0.0f) {
@@ -835,15 +852,16 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
 #pragma unroll
                             for (int f = 0; f < F; ++f)
                                 rm[f] = rg_row<QC_DEG_LOW, MODE, Z>(p, (size_t)blockIdx.x * F + f, ly, j);
-                            if constexpr (CIRC) row_update_circ<QC_DEG_LOW, MODE, F>(idx, sL, lstride, rm, cr);
-                            else row_update<QC_DEG_LOW, MODE, ALGO, CLIP, F>(idx, sL, lstride, rm, r_cap, lp_cap, wl);
+                            if constexpr (CIRC) row_update_circ<QC_DEG_LOW, MODE, F, RowMsgGlobal<QC_DEG_LOW, MODE>, false, SC>(idx, sL, lstride, rm, cr);
+                            else row_update<QC_DEG_LOW, MODE, ALGO, CLIP, F, RowMsgGlobal<QC_DEG_LOW, MODE>, false, false, SC>(
+                                idx, sL, lstride, rm, r_cap, lp_cap, wl);
                         } else if constexpr (PAIR)
                             row_update_pair<QC_DEG_LOW, MODE>(idx, sL, msg.r3[ly & 3]);
                         else if constexpr (CIRC)
-                            row_update_circ<QC_DEG_LOW, MODE, F, RowMsg<QC_DEG_LOW, MODE>, OT>(
+                            row_update_circ<QC_DEG_LOW, MODE, F, RowMsg<QC_DEG_LOW, MODE>, OT, SC>(
                                 idx, sL, lstride, msg.r3[ly & 3][rho], cr);
                         else
-                            row_update<QC_DEG_LOW, MODE, ALGO, CLIP, F, RowMsg<QC_DEG_LOW, MODE>, OT>(
+                            row_update<QC_DEG_LOW, MODE, ALGO, CLIP, F, RowMsg<QC_DEG_LOW, MODE>, OT, false, SC>(
                                 idx, sL, lstride, msg.r3[ly & 3][rho], r_cap, lp_cap, wl);
                     } else {
                         int idx[D];
@@ -859,15 +877,16 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
 #pragma unroll
                             for (int f = 0; f < F; ++f)
                                 rm[f] = rg_row<D, MODE, Z>(p, (size_t)blockIdx.x * F + f, ly, j);
-                            if constexpr (CIRC) row_update_circ<D, MODE, F>(idx, sL, lstride, rm, cr);
-                            else row_update<D, MODE, ALGO, CLIP, F>(idx, sL, lstride, rm, r_cap, lp_cap, wl);
+                            if constexpr (CIRC) row_update_circ<D, MODE, F, RowMsgGlobal<D, MODE>, false, SC>(idx, sL, lstride, rm, cr);
+                            else row_update<D, MODE, ALGO, CLIP, F, RowMsgGlobal<D, MODE>, false, false, SC>(
+                                idx, sL, lstride, rm, r_cap, lp_cap, wl);
                         } else if constexpr (PAIR)
                             row_update_pair<D, MODE>(idx, sL, msg.rD[(ly - 4) & 7]);
                         else if constexpr (CIRC)
-                            row_update_circ<D, MODE, F, RowMsg<D, MODE>, OT>(idx, sL, lstride,
+                            row_update_circ<D, MODE, F, RowMsg<D, MODE>, OT, SC>(idx, sL, lstride,
                                                                             msg.rD[(ly - 4) & 7][rho], cr);
                         else
-                            row_update<D, MODE, ALGO, CLIP, F, RowMsg<D, MODE>, OT>(
+                            row_update<D, MODE, ALGO, CLIP, F, RowMsg<D, MODE>, OT, false, SC>(
                                 idx, sL, lstride, msg.rD[(ly - 4) & 7][rho], r_cap, lp_cap, wl);
                     }
                 }
@@ -891,7 +910,8 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
 #pragma unroll
                         for (int f = 0; f < F; ++f)
                             rm[f] = rg_row<D, MODE, Z>(p, (size_t)blockIdx.x * F + f, ly, j);
-                        row_update<D, MODE, ALGO, CLIP, F>(idx, sL, lstride, rm, r_cap, lp_cap, wl);
+                        row_update<D, MODE, ALGO, CLIP, F, RowMsgGlobal<D, MODE>, false, false, SC>(
+                            idx, sL, lstride, rm, r_cap, lp_cap, wl);
                     }
                     __syncthreads();
                 }
@@ -1059,6 +1079,14 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                 if (p.iters_out) p.iters_out[fid[f]] = it[f];
                 if (p.synd_out) p.synd_out[fid[f]] = (int32_t)sf;
                 if (p.be_out) p.be_out[fid[f]] = (int32_t)be;
+            }
+            if constexpr (SC) {
+                if (it[f] >= SCALED_CHECK_FROM) {
+                    const SV L(sL, f, lstride);
+                    bool far = false;
+                    for (int i = tid; i < N; i += T) far |= !(fabsf(L.ld(i)) < SCALED_LIMIT);
+                    if (far) p.tally[T_OUT_OF_RANGE] = 1ull;
+                }
             }
             if (p.post_out) {
                 const SV L(sL, f, lstride);

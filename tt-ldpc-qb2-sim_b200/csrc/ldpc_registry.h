@@ -24,7 +24,12 @@ struct QcKey {
 struct QcEntry {
     QcKey key;
     const void* fn;  // __global__ void (const QcParams)
+    bool scaled;     // decodes at LLR_SCALE: only for channels qc_scaled_ok accepts
 };
+// Which variants are built scaled: all but the plain shapes, which serve the channels outside its range.
+constexpr bool qc_scaled(int mode, int algo, bool clip, bool ext) {
+    return !ext && !clip && mode != 2 /* STORE_FP16 */ && (algo == 0 /* ALGO_AMIN */ || algo == 3 /* ALGO_CIRC */);
+}
 
 struct QcTable {
     const QcEntry* entries;
@@ -61,39 +66,52 @@ const QcTable* qc_tables();
 #define LDPC_QC_ENTRY(Z, D, R, F, MODE, ALGO, CLIP, EXT) LDPC_QC_ENTRY_B(Z, D, R, F, MODE, ALGO, CLIP, EXT, 0)
 #define LDPC_QC_ENTRY_B(Z, D, R, F, MODE, ALGO, CLIP, EXT, B)                  \
     {{Z, D, R, F, MODE, ALGO, CLIP, EXT, B, 0},                                \
-     reinterpret_cast<const void*>(&::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B>)}
+     reinterpret_cast<const void*>(                                            \
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, false, false, -1, false, \
+                                       (B > 0) && ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)>),             \
+     (B > 0) && ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)}
 #define LDPC_QC_ENTRY_G(Z, D, R, F, MODE, ALGO, CLIP, EXT, B)                  \
     {{Z, D, R, F, MODE, ALGO, CLIP, EXT, B, 1},                                \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, true>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, true, false, -1, false, \
+                                       (B > 0) && ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)>),             \
+     (B > 0) && ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)}
 
 // Layout 5: the global-message kernel with the layer descriptors of fixed-table code FIX compiled in.
 #define LDPC_QC_ENTRY_GF(Z, D, R, F, MODE, ALGO, CLIP, EXT, B, FIX)           \
     {{Z, D, R, F, MODE, ALGO, CLIP, EXT, B, 5},                                \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, true, false, FIX>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, true, false, FIX, false, \
+                                       ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)>),                        \
+     ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)}
 
 // Layout 6: messages in registers with the layer descriptors of fixed-table code FIX compiled in.
 #define LDPC_QC_ENTRY_RF(Z, D, R, F, MODE, ALGO, CLIP, EXT, B, FIX)           \
     {{Z, D, R, F, MODE, ALGO, CLIP, EXT, B, 6},                                \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, false, false, FIX>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, false, false, FIX, false, \
+                                       ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)>),                        \
+     ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)}
 
 // Layout 7: the global-message kernel with its degree-D layers in a loop that is not unrolled.
 #define LDPC_QC_ENTRY_GR(Z, D, R, F, MODE, ALGO, CLIP, EXT, B)                 \
     {{Z, D, R, F, MODE, ALGO, CLIP, EXT, B, 7},                                \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, true, false, -1, true>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, true, false, -1, true, \
+                                       ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)>),                        \
+     ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)}
 
 #define LDPC_QC_ENTRY_OT(Z, D, R, F, MODE, ALGO, CLIP, EXT, B)                 \
     {{Z, D, R, F, MODE, ALGO, CLIP, EXT, B, 2},                                \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, false, true>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, CLIP, EXT, B, false, false, true, -1, false, \
+                                       ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)>),                        \
+     ::ldpcb200::qc_scaled(MODE, ALGO, CLIP, EXT)}
 
 #define LDPC_QC_ENTRY_PAIR(Z, D, MODE, EXT, B)                                 \
     {{Z, D, 1, 2, MODE, ::ldpcb200::ALGO_AMIN, 0, EXT, B, 0},                  \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, 1, 2, MODE, ::ldpcb200::ALGO_AMIN, false, EXT, B, true>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, 1, 2, MODE, ::ldpcb200::ALGO_AMIN, false, EXT, B, true>), false}
 
 // Layout 5 or 7 with the clips compiled in for a variant without clips: with infinite caps they leave every
 // value but NaN as it is, and a NaN posterior (from a NaN channel LLR) becomes -inf, as in the general kernel
@@ -101,11 +119,11 @@ const QcTable* qc_tables();
 #define LDPC_QC_ENTRY_GF_NAN(Z, D, R, F, MODE, ALGO, EXT, B, FIX)             \
     {{Z, D, R, F, MODE, ALGO, 0, EXT, B, 5},                                   \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, true, EXT, B, false, true, false, FIX>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, true, EXT, B, false, true, false, FIX>), false}
 #define LDPC_QC_ENTRY_GR_NAN(Z, D, R, F, MODE, ALGO, EXT, B)                   \
     {{Z, D, R, F, MODE, ALGO, 0, EXT, B, 7},                                   \
      reinterpret_cast<const void*>(                                            \
-         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, true, EXT, B, false, true, false, -1, true>)}
+         &::ldpcb200::qc_decode_kernel<Z, D, R, F, MODE, ALGO, true, EXT, B, false, true, false, -1, true>), false}
 
 #define LDPC_QC_DEFAULTS(name)                                                           \
     namespace {                                                                          \
