@@ -93,3 +93,58 @@ def test_circulant_decoder(gpu, K, storage):
                                                     algo=capi.ALGO_CIRC)
                     assert (r.bit_errors, r.frame_errors, r.iter_sum, r.unconverged) == \
                         (t.bit_errors, t.frame_errors, t.iter_sum, t.unconverged), (num, stop, sh, n)
+
+
+def _general(code, llr, **kw):
+    """The general kernel on the same matrix: four columns fewer punctured, with LLR 0."""
+    with capi.Decoder(code.row_matrix(), code.N, code.P - 4) as g:
+        assert g.kind == capi.KERNEL_GENERAL
+        post, it, sf, _, _ = g.decode_llr(np.concatenate([llr, np.zeros((len(llr), 4), np.float32)], 1), **kw)
+    return post, it, sf
+
+
+def _static(code, llr, p):
+    import torch
+    x = torch.from_numpy(llr).cuda()
+    post = torch.empty(len(llr), code.N, device="cuda")
+    it, sf = (torch.empty(len(llr), dtype=torch.int32, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    capi.decode_llr_static(code.row_matrix(), code.N, code.P, p, x.data_ptr(), len(llr), post.data_ptr(), it.data_ptr(),
+                           sf.data_ptr())
+    return post.cpu().numpy(), it.cpu().numpy(), sf.cpu().numpy()
+
+
+@pytest.mark.parametrize("K,rate", ar4ja.ALL_CODES)
+@pytest.mark.parametrize("storage", ["fp32", "bf16"])
+def test_caller_llrs(gpu, K, rate, storage):
+    """Posterior bits, iterations and syndromes of caller-supplied LLRs (host and device entry) against the
+    general kernel: frames in range (zeros and the smallest and largest scalable values among them), then
+    with one LLR out of range, for which the call runs unscaled."""
+    code = ar4ja.make_code(K, rate)
+    mu, sigma = capi.channel_mu_sigma(code.N, code.n_checks, code.P, TH[rate] + 0.4)
+    llr = (mu + sigma * np.random.default_rng(8).standard_normal((6, code.n_tx))).astype(np.float32)
+    llr[1, ::7] = 0.0
+    llr[2, 5], llr[2, 6], llr[3, 7], llr[4, 9] = -0.0, 2.0 ** -70, 1048575.0, -1048575.0
+    kw = dict(max_iter=44, storage=storage)
+    with capi.Decoder.from_code(code) as d:
+        for extra in (None, 2.0 ** -130, 1048576.0, 1e30, -3e-39):
+            if extra is not None:
+                llr[5, 11] = extra
+            want = _general(code, llr, **kw)
+            for got in (d.decode_llr(llr, **kw)[:3], _static(code, llr, d.params(**kw))):
+                assert np.array_equal(got[0].view(np.uint32), want[0].view(np.uint32)), extra
+                assert np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2]), extra
+
+
+def test_large_caller_calls_out_of_range(gpu):
+    """A call through the chunked copies with one LLR out of range in its last frame: decoded again, the
+    same as in range for every other frame."""
+    code = ar4ja.make_code(1024, "1/2")
+    mu, sigma = capi.channel_mu_sigma(code.N, code.n_checks, code.P, 2.0)
+    llr = (mu + sigma * np.random.default_rng(9).standard_normal((17000, code.n_tx))).astype(np.float32)
+    with capi.Decoder.from_code(code) as d:
+        a = d.decode_llr(llr, max_iter=30, storage="fp32", want_post=False)
+        llr[-1, 0] = 3e30
+        b = d.decode_llr(llr, max_iter=30, storage="fp32", want_post=False)
+    assert all(np.array_equal(x[:-1], y[:-1]) for x, y in zip(a[1:4], b[1:4]))
+    assert b[4].frames == 17000 and b[4].iter_sum == b[1].sum()

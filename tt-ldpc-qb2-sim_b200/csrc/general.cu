@@ -499,9 +499,9 @@ int launch_general(GeneralCode* g, const ldpc_run_params* p, bool ext, uint32_t 
 //
 // A matrix with the quasi-cyclic structure runs on the QC kernel (run_static_qc): its messages stay in
 // registers or take one slot per CTA, it needs no row schedule, and a frame has a whole CTA instead of one
-// warp.  Its variants with the clips compiled in are used whatever the clips (with infinite caps they change
-// only a NaN posterior, to -inf, as the general kernel does).  4001 frames r1/2 K=1024 bf16 2.0 dB with
-// posteriors: 3.00 ms on the general kernel (1.41 of them its schedule), 0.41.
+// warp.  LLRs in range run on the scaled kernels; all else on the variants with the clips compiled in, whatever
+// the clips (with infinite caps they change only a NaN posterior, to -inf, as the general kernel does).  4001 frames r1/2 K=1024 bf16 2.0 dB with
+// posteriors: 3.00 ms on the general kernel (1.41 of them its schedule), 0.29.
 //
 // Scratch layout of the general kernel (LDPC_STATIC_SCRATCH_BYTES, 256-byte aligned regions):
 //   [0, 256)           frame-claim counter (u32) and tallies (TALLY_WORDS x u64)
@@ -636,7 +636,7 @@ constexpr uint64_t kStaticLaunchFrames = 1ull << 31;
 // the alignment of d_llr (the kernel reads four LLRs at a time) ask for the general kernel.
 static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const float* d_llr, uint64_t n, float* d_post,
                          int32_t* d_iters, int32_t* d_synd, int32_t* d_be, ldpc_tally* out, unsigned char* base, int dev,
-                         cudaStream_t stream, std::string& err) {
+                         cudaStream_t stream, std::string& err, bool scaled) {
     const int N = h->n_vars, P = h->n_punct;
     QcStructure s = {};
     if (!n || (N - P) % 32 || reinterpret_cast<uintptr_t>(d_llr) % 16 ||
@@ -652,7 +652,7 @@ static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const f
         cudaGetLastError();
         return LDPC_ENOTSUP;
     }
-    // the default shape; a shape with messages in global memory only if the scratch holds a slot for every
+    // the default shape (unscaled: its variant with clips); a shape with messages in global memory only if the scratch holds a slot for every
     // resident CTA, or if there is no other
     const void* fn = nullptr;
     int sh[4];
@@ -660,8 +660,9 @@ static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const f
     uint64_t grid = 0;
     for (int scratch = 1; scratch >= 0; --scratch) {
         int t[4];
-        const void* f = qc_default(s.Z, s.D, s.fix, p->storage, p->algo, 1, 1, most, scratch != 0, t);
-        if (!f || t[1] != 1 || (!scratch && qc_shape_in_scratch(t[3]))) continue;
+        const QcEntry* entry = qc_default(s.Z, s.D, s.fix, p->storage, p->algo, !scaled, 1, most, scratch != 0, t, scaled);
+        if (!entry || entry->scaled != scaled || t[1] != 1 || (!scratch && qc_shape_in_scratch(t[3]))) continue;
+        const void* f = entry->fn;
         const size_t sm = qc_smem_bytes(N, s.Z, s.D, t[0], t[1], t[3], p->storage);
         int per_sm = 0;
         if ((sm > 48 * 1024 && cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) ||
@@ -712,6 +713,7 @@ static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const f
         err = std::string("static decode: ") + cudaGetErrorString(e);
         return LDPC_EIO;
     }
+    if (t[T_OUT_OF_RANGE]) return LDPC_ENOTSUP;  // scaled only: the caller decodes the frames again unscaled
     tally_out(t, out);
     return 0;
 }
@@ -729,12 +731,15 @@ int decode_llr_static(const ldpc_matrix* h, const ldpc_run_params* p, const floa
     if (p->max_iter < 0 || p->storage < 0 || p->storage > 2 || p->algo < 0 || p->algo > 1)
         return sfail(LDPC_EINVAL, err, "bad run parameters");
     int maxdeg = 0;
-    for (int64_t i = 0; i < (int64_t)M * dmax; ++i) {
-        const int32_t c = h->rows[i];
-        if (c < -1 || c >= N) return sfail(LDPC_EINVAL, err, "edge index out of bounds");
-        if (c >= 0 && i % dmax > 0 && h->rows[i - 1] < 0)
-            return sfail(LDPC_EINVAL, err, "edge after the -1 that ends its row");
-        if (c >= 0) maxdeg = std::max(maxdeg, (int)(i % dmax) + 1);
+    for (int m = 0; m < M; ++m) {
+        const int32_t* row = h->rows + (size_t)m * dmax;
+        for (int e = 0; e < dmax; ++e) {
+            const int32_t c = row[e];
+            if (c < -1 || c >= N) return sfail(LDPC_EINVAL, err, "edge index out of bounds");
+            if (c < 0) continue;
+            if (e > 0 && row[e - 1] < 0) return sfail(LDPC_EINVAL, err, "edge after the -1 that ends its row");
+            maxdeg = std::max(maxdeg, e + 1);
+        }
     }
     const int dt = maxdeg <= 6 ? 6 : maxdeg <= 8 ? 8 : maxdeg <= 20 ? 20 : 32;
     const int dtc = gen_dtc(dt);
@@ -791,8 +796,12 @@ int decode_llr_static(const ldpc_matrix* h, const ldpc_run_params* p, const floa
         cudaGetLastError();
         return sfail(LDPC_ENOTSUP, err, "frame too large for shared memory");
     }
-    const int qc = run_static_qc(h, p, d_llr, (uint64_t)n, d_post, d_iters, d_synd, d_be, out, base, dev, stream, err);
-    if (qc != LDPC_ENOTSUP) return qc;
+    const bool clip = p->l_max > 0.0f || p->r_max > 0.0f || p->l_post_max > 0.0f;
+    for (int scaled = !clip && p->algo == ALGO_AMIN && p->max_iter <= 10000; scaled >= 0; --scaled) {
+        const int qc = run_static_qc(h, p, d_llr, (uint64_t)n, d_post, d_iters, d_synd, d_be, out, base, dev, stream, err,
+                                     scaled != 0);
+        if (qc != LDPC_ENOTSUP) return qc;
+    }
     int per_sm = 0, n_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * nw, smem) != cudaSuccess ||
         cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || per_sm <= 0) {

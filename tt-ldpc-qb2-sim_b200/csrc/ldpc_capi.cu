@@ -69,7 +69,9 @@ static const QcEntry* find_qc(const QcKey& k, bool scaled) {
 // Whether the scaled kernels may decode a simulated channel: LLR mean and deviation between 2^-10 and 2^12 (or 0),
 // i.e. an Eb/N0 between about -30 and 30 dB, and at most 10000 iterations; values then stay far inside the
 // range LLR_SCALE leaves, and the kernel checks long frames all the same.
-static bool qc_scaled_ok(const ldpc_run_params* p) {
+// Caller-supplied LLRs (ext) are checked by the kernel.
+static bool qc_scaled_ok(const ldpc_run_params* p, bool ext) {
+    if (ext) return p->max_iter <= 10000;
     auto in = [](float v) { return v == 0.0f || (v >= 9.765625e-4f && v <= 4096.0f); };
     const bool snr = p->ebn0_hi_db > p->ebn0_lo_db;
     return p->max_iter <= 10000 &&
@@ -114,7 +116,7 @@ struct ldpc_handle {
     static constexpr size_t kSmallLlr = (kCounterBytes + kSmallBytes + 255) / 256 * 256;
     static constexpr size_t kSmallLlr16 = kSmallLlr + kSmallBytes;
     static constexpr size_t kIoBytes = kSmallLlr16 + kSmallBytes / 2;
-    unsigned char* h_small = nullptr;  // pinned, on first use: tally and outputs, then LLRs
+    unsigned char* h_small = nullptr;  // pinned: the tally, a small call's outputs, its LLRs
     static constexpr size_t kSmallHostLlr = (TALLY_WORDS * 8 + kSmallBytes + 255) / 256 * 256;
     float* d_llr = nullptr;
     size_t llr_cap = 0;
@@ -131,7 +133,7 @@ struct ldpc_handle {
     bool w_row = false;
     // settings of LDPC_ALGO_CIRC runs (default: the circulant engine on silicon)
     ldpc_circ_config circ{LDPC_CIRC_SFPU, LDPC_CIRC_STOP_GENIE, 0.9375f, 0};
-    unsigned long long* h_tally = nullptr;  // pinned
+    unsigned long long* h_tally = nullptr;  // the start of h_small
     int64_t launches = 0;
     // ldpc_decode_llr: a copy stream and an event that let the decoding of one chunk of frames
     // overlap the host->device copy of the next (created on first use)
@@ -244,7 +246,6 @@ extern "C" void ldpc_destroy(ldpc_handle* h) {
     cudaFree(h->d_wtab);
     cudaFree(h->d_wtab_row);
     free_general(&h->gen);
-    if (h->h_tally) cudaFreeHost(h->h_tally);
     if (h->h_small) cudaFreeHost(h->h_small);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
@@ -308,8 +309,9 @@ extern "C" int ldpc_create(const ldpc_matrix* m, int device, ldpc_handle** out) 
         cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
         return bail(fail(LDPC_EIO, "stream/event creation failed"));
     if (cudaMalloc(&h->d_io, ldpc_handle::kIoBytes) != cudaSuccess ||
-        cudaMallocHost(&h->h_tally, TALLY_WORDS * sizeof(unsigned long long)) != cudaSuccess)
+        cudaMallocHost(&h->h_small, ldpc_handle::kSmallHostLlr + ldpc_handle::kSmallBytes) != cudaSuccess)
         return bail(fail(LDPC_ENOMEM, "device allocation failed"));
+    h->h_tally = reinterpret_cast<unsigned long long*>(h->h_small);
     h->d_work = reinterpret_cast<unsigned int*>(h->d_io);
     h->d_hist = reinterpret_cast<unsigned long long*>(h->d_io + 64);
     h->d_snr = h->d_hist + h->hist_bins;
@@ -388,12 +390,11 @@ static const QcEntry* find_shape(const ldpc_handle* h, int storage, int algo, in
 // built, else the first shape built for it (e.g. the global-message kernel of a K = 16384 code).
 // scratch = false leaves out the lines that need a message scratch.
 namespace ldpcb200 {
-const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4],
+const QcEntry* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4],
                        bool scaled) {
-    auto built = [&](int R, int F, int B, int G) -> const void* {
+    auto built = [&](int R, int F, int B, int G) -> const QcEntry* {
         if ((G == 5 || G == 6) && fix < 0) return nullptr;  // compiled-in descriptors of another code
-        const QcEntry* e = find_qc(QcKey{Z, D, R, F, storage, algo, clip, ext, B, G}, scaled);
-        return e ? e->fn : nullptr;
+        return find_qc(QcKey{Z, D, R, F, storage, algo, clip, ext, B, G}, scaled);
     };
     for (int own = 1; own >= 0; --own)
         for (const QcDefaults* t = qc_defaults(); t; t = t->next)
@@ -402,14 +403,14 @@ const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, i
                 if (d.Z != Z || d.D != D || d.mode != storage || d.algo != (own ? algo : -1) || n < d.min_frames ||
                     (!scratch && qc_shape_in_scratch(d.G)))
                     continue;
-                if (const void* fn = built(d.R, d.F, d.B, d.G)) {
+                if (const QcEntry* e = built(d.R, d.F, d.B, d.G)) {
                     s[0] = d.R; s[1] = d.F; s[2] = d.B; s[3] = d.G;
-                    return fn;
+                    return e;
                 }
             }
-    if (const void* fn = built(1, 1, 0, 0)) {
+    if (const QcEntry* e = built(1, 1, 0, 0)) {
         s[0] = 1; s[1] = 1; s[2] = 0; s[3] = 0;
-        return fn;
+        return e;
     }
     for (const QcTable* t = qc_tables(); t; t = t->next)
         for (int i = 0; i < t->count; ++i) {
@@ -417,7 +418,7 @@ const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, i
             if (k.Z == Z && k.D == D && k.mode == storage && k.algo == algo && k.clip == clip && k.ext == ext &&
                 ((k.G != 5 && k.G != 6) || fix >= 0) && (scaled || !t->entries[i].scaled)) {
                 s[0] = k.R; s[1] = k.F; s[2] = k.B; s[3] = k.G;
-                return t->entries[i].fn;
+                return &t->entries[i];
             }
         }
     return nullptr;
@@ -662,7 +663,7 @@ static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const QcEn
 static int prepare_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32_t n, uint64_t first,
                       const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be,
                       double grid_frac, QcLaunch* out, bool scaled) {
-    scaled = scaled && !ext && qc_scaled_ok(p);
+    scaled = scaled && qc_scaled_ok(p, ext);
     const bool clip = p->l_max > 0.0f || p->r_max > 0.0f || p->l_post_max > 0.0f;
     int sh[4];
     bool chosen = false, scratch = true;
@@ -1035,7 +1036,7 @@ static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64
             if (sh[3] != GEN_LAYOUT_WARP)
                 rc = launch_general_step(&h->gen, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be,
                                          h->d_tally, h->d_hist, h->hist_bins, h->d_work, h->n_sm, h->stream, g_err,
-                                         h->d_snr, scaled && qc_scaled_ok(p));
+                                         h->d_snr, scaled && !ext && qc_scaled_ok(p, ext));
             if (rc == LDPC_ENOTSUP)
                 rc = launch_general(&h->gen, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be, h->d_tally,
                                     h->d_hist, h->hist_bins, h->d_work, h->n_sm, h->stream, g_err, h->d_snr);
@@ -1073,25 +1074,14 @@ static bool host_memory(const void* p, bool* pageable = nullptr) {
     return a.type == cudaMemoryTypeUnregistered || a.type == cudaMemoryTypeHost;
 }
 
-static int small_alloc(ldpc_handle* h) {
-    if (!h->h_small &&
-        cudaMallocHost(&h->h_small, ldpc_handle::kSmallHostLlr + ldpc_handle::kSmallBytes) != cudaSuccess) {
-        cudaGetLastError();
-        h->h_small = nullptr;
-        return fail(LDPC_ENOMEM, "pinned buffer allocation failed");
-    }
-    return 0;
-}
-
 // A call whose LLRs and outputs take at most kSmallBytes each: one stream, one pinned buffer, one copy each way
 // (the outputs follow the tally on the device), the caller's arrays read and written by the host.  One frame
 // r1/2 K=1024 fp32 with posteriors, whole call: 59 us, 113 with the copies of the large path (a second
-// stream, one copy per output into pageable memory); its first call on a handle 3 ms, 69 to 80 with the ring.
+// stream, one copy per output into pageable memory); its first call on a handle 0.13 ms, 37 to 80 with the ring.
 static int decode_small(ldpc_handle* h, const ldpc_run_params* p, const void* llr, int elem, size_t n, float* post,
                         int32_t* iters, int32_t* synd_fail, int32_t* bit_errors, ldpc_tally* out) {
     using H = ldpc_handle;
     int rc;
-    if ((rc = small_alloc(h))) return rc;
     const size_t ntx = (size_t)(h->N - h->P), in_bytes = n * ntx * elem;
     unsigned char* h_llr = h->h_small + H::kSmallHostLlr;
     float* d_llr = reinterpret_cast<float*>(h->d_io + H::kSmallLlr);
@@ -1107,11 +1097,17 @@ static int decode_small(ldpc_handle* h, const ldpc_run_params* p, const void* ll
     int32_t* d_it = reinterpret_cast<int32_t*>(h->d_io + H::kCounterBytes);
     int32_t *d_sf = d_it + n, *d_be = d_sf + n;
     float* d_post = reinterpret_cast<float*>(d_be + n);
-    if ((rc = run_frames(h, p, true, n, d_llr, post ? d_post : nullptr, d_it, d_sf, d_be))) return rc;
     const size_t post_bytes = post ? n * h->N * sizeof(float) : 0;
-    CU(cudaMemcpyAsync(h->h_small, h->d_tally, TALLY_WORDS * 8 + 3 * n * sizeof(int32_t) + post_bytes,
-                       cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaStreamSynchronize(h->stream));
+    // (scaled; again on the unscaled kernels if the LLRs are out of the scaled ones' range)
+    for (int scaled = 1; scaled >= 0; --scaled) {
+        if ((rc = run_frames(h, p, true, n, d_llr, post ? d_post : nullptr, d_it, d_sf, d_be, nullptr, kMaxLaunchFrames,
+                             scaled != 0)))
+            return rc;
+        CU(cudaMemcpyAsync(h->h_small, h->d_tally, TALLY_WORDS * 8 + 3 * n * sizeof(int32_t) + post_bytes,
+                           cudaMemcpyDeviceToHost, h->stream));
+        CU(cudaStreamSynchronize(h->stream));
+        if (!reinterpret_cast<const unsigned long long*>(h->h_small)[T_OUT_OF_RANGE]) break;
+    }
     const unsigned char* o = h->h_small + TALLY_WORDS * 8;
     if (iters) memcpy(iters, o, n * sizeof(int32_t));
     if (synd_fail) memcpy(synd_fail, o + n * sizeof(int32_t), n * sizeof(int32_t));
@@ -1149,6 +1145,37 @@ static int unstage_d2h(ldpc_handle* h, char* dst, const char* src, size_t bytes)
         got += b;
     }
     return 0;
+}
+
+// The outputs of a large call to the caller's arrays, and the tally.
+static int host_outputs(ldpc_handle* h, size_t nb, bool plain, float* post, int32_t* iters, int32_t* synd_fail,
+                        int32_t* bit_errors, ldpc_tally* out) {
+    int rc;
+    if (!nb) return read_tally(h, out);
+    int32_t *d_it = h->d_frame_out, *d_sf = d_it + nb, *d_be = d_sf + nb;
+    bool ring = false;
+    if (post && host_memory(post, &ring) && ring) {
+        if ((rc = unstage_d2h(h, reinterpret_cast<char*>(post), reinterpret_cast<const char*>(h->d_post),
+                              nb * h->N * sizeof(float))))
+            return rc;
+    } else if (post) {
+        CU(cudaMemcpyAsync(post, h->d_post, nb * h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+    }
+    // the per-frame counts: one copy into the pinned buffer where they fit, else one per array
+    if (plain && 3 * nb * sizeof(int32_t) <= ldpc_handle::kSmallBytes) {
+        unsigned char* buf = h->h_small + TALLY_WORDS * 8;
+        CU(cudaMemcpyAsync(buf, d_it, 3 * nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+        if ((rc = read_tally(h, out))) return rc;
+        const int32_t* o = reinterpret_cast<const int32_t*>(buf);
+        if (iters) memcpy(iters, o, nb * sizeof(int32_t));
+        if (synd_fail) memcpy(synd_fail, o + nb, nb * sizeof(int32_t));
+        if (bit_errors) memcpy(bit_errors, o + 2 * nb, nb * sizeof(int32_t));
+        return 0;
+    }
+    if (iters) CU(cudaMemcpyAsync(iters, d_it, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    if (synd_fail) CU(cudaMemcpyAsync(synd_fail, d_sf, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    if (bit_errors) CU(cudaMemcpyAsync(bit_errors, d_be, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
+    return read_tally(h, out);
 }
 
 // ldpc_decode_llr and ldpc_decode_llr_bf16: caller LLRs of `elem` bytes each (4: fp32, 2: bf16).
@@ -1195,31 +1222,13 @@ static int decode_host(ldpc_handle* h, const ldpc_run_params* p, const void* llr
     if ((rc = run_frames(h, &q, true, nb, h->d_llr, post ? h->d_post : nullptr, d_it, d_sf, d_be,
                          nb ? &hin : nullptr, chunk)))
         return rc;
-    if (nb) {
-        bool ring = false;
-        if (post && host_memory(post, &ring) && ring) {
-            if ((rc = unstage_d2h(h, reinterpret_cast<char*>(post), reinterpret_cast<const char*>(h->d_post),
-                                  nb * h->N * sizeof(float))))
-                return rc;
-        } else if (post) {
-            CU(cudaMemcpyAsync(post, h->d_post, nb * h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-        }
-        // the per-frame counts: one copy into the pinned buffer where they fit, else one per array
-        if (plain && 3 * nb * sizeof(int32_t) <= ldpc_handle::kSmallBytes) {
-            if ((rc = small_alloc(h))) return rc;
-            CU(cudaMemcpyAsync(h->h_small, d_it, 3 * nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-            if ((rc = read_tally(h, out))) return rc;
-            const int32_t* o = reinterpret_cast<const int32_t*>(h->h_small);
-            if (iters) memcpy(iters, o, nb * sizeof(int32_t));
-            if (synd_fail) memcpy(synd_fail, o + nb, nb * sizeof(int32_t));
-            if (bit_errors) memcpy(bit_errors, o + 2 * nb, nb * sizeof(int32_t));
-            return 0;
-        }
-        if (iters) CU(cudaMemcpyAsync(iters, d_it, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-        if (synd_fail) CU(cudaMemcpyAsync(synd_fail, d_sf, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-        if (bit_errors) CU(cudaMemcpyAsync(bit_errors, d_be, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    }
-    return read_tally(h, out);
+    if ((rc = host_outputs(h, nb, plain, post, iters, synd_fail, bit_errors, out))) return rc;
+    if (!nb || !h->h_tally[T_OUT_OF_RANGE]) return 0;
+    // the LLRs, now on the device, are out of the scaled kernels' range
+    if ((rc = run_frames(h, &q, true, nb, h->d_llr, post ? h->d_post : nullptr, d_it, d_sf, d_be, nullptr, kMaxLaunchFrames,
+                         false)))
+        return rc;
+    return host_outputs(h, nb, plain, post, iters, synd_fail, bit_errors, out);
 }
 
 extern "C" int ldpc_decode_llr(ldpc_handle* h, const ldpc_run_params* p, const float* llr, int64_t n,

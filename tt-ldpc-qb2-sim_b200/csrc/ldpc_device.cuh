@@ -135,7 +135,8 @@ __device__ __forceinline__ float amin_step_scaled(float m, float a) {
 // A scaled frame's magnitudes are checked where they could have grown: frames of at least this many iterations,
 // against 2^40.  One beyond it makes the host decode the call again on the unscaled kernels.
 constexpr int SCALED_CHECK_FROM = 40;
-constexpr float SCALED_LIMIT = 9.765625e-4f;  // 2^40 scaled
+constexpr float SCALED_LIMIT = 9.765625e-4f;            // 2^40 scaled
+constexpr float SCALED_LLR_LIMIT = 9.3132257461547852e-10f;  // 2^20 scaled: caller-supplied channel LLRs
 
 // The circulant engine's min* (tests/test_circulant_dma_stepper.cpp:39-54 and
 // engines/tile_matrix_4cw/sfpi_host_emu.h:590-607): max(min(a, b) - max(c1 + k1 d, c2 + k2 d, 0), 0)

@@ -88,7 +88,8 @@ struct QcStructure {
     int32_t blk_off[QC_LAYERS][QC_DMAX], shift[QC_LAYERS][QC_DMAX];
 };
 bool qc_structure(const int32_t* rows, int N, int M, int P, int dmax, QcStructure* out);
-const void* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4],
+struct QcEntry;
+const QcEntry* qc_default(int Z, int D, int fix, int storage, int algo, int clip, int ext, uint32_t n, bool scratch, int s[4],
                        bool scaled = false);
 void qc_message_layout(QcParams* qp, int Z, int D);
 size_t qc_smem_bytes(int N, int Z, int D, int R, int F, int G, int storage);
@@ -652,8 +653,9 @@ __device__ __forceinline__ int qc_shift(const QcParams& p, int l, int e) {
 // words (T * (12 + 8 D) words); one row per thread.
 // FIX: >= 0 for the descriptors of a known code compiled in (layouts 5 and 6; the host offers them
 // only for a matrix whose descriptors are those).
-// SC: the frames are decoded at LLR_SCALE (the simulation of Approximate-Min* or the circulant engine's decoder,
-// fp32 or bf16 storage, no clips): the same tallies, one instruction less per min* step.
+// SC: the frames are decoded at LLR_SCALE (Approximate-Min*, or the simulation of the circulant engine's decoder;
+// fp32 or bf16 storage, no clips): the same values but for the scale, one instruction less per min* step.  A
+// caller's LLR that does not scale exactly or is 2^20 or more (or NaN) is reported in the tally.
 // ROLL (layout 7, global messages only): the eight degree-D layers run as one loop that is not
 // unrolled, each row's descriptors read from the kernel parameters by layer index.  The unrolled
 // body of a degree-18 code is tens of KB of instructions; with one-warp CTAs whose warps are
@@ -671,8 +673,8 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
     static_assert(!OT || (!PAIR && !RG && R == 1), "the offset table is built for one row per thread");
     static_assert(FIX < 0 || (!OT && !PAIR && FIX < QC_FIXED_COUNT), "compiled-in descriptors: no offset table");
     constexpr bool CIRC = ALGO == ALGO_CIRC;
-    static_assert(!SC || (!EXT && !CLIP && !PAIR && MODE != STORE_FP16 && (CIRC || ALGO == ALGO_AMIN)),
-                  "scaled decoding: the simulation, no clips, no fp16 messages");
+    static_assert(!SC || (!CLIP && !PAIR && MODE != STORE_FP16 && (ALGO == ALGO_AMIN || (CIRC && !EXT))),
+                  "scaled decoding: no clips, no fp16 messages");
     static_assert(!ROLL || (RG && FIX < 0 && !CIRC), "the rolled layer loop: global messages, parameter descriptors");
     static_assert(!CIRC || (D == 6 && !CLIP && !PAIR), "the circulant engine's decoder: degrees 3 and 6, no clips");
     using SV = SlotView<MODE, PAIR>;
@@ -757,6 +759,7 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                 const int nq = p.n_tx >> 2;
                 if (EXT) {
                     const float4* src = reinterpret_cast<const float4*>(p.llr_in + (size_t)fid[f] * p.n_tx);
+                    bool far = false;
                     for (int qd = tid; qd < nq; qd += T) {
                         const float4 v4 = src[qd];
                         float v[4] = {v4.x, v4.y, v4.z, v4.w};
@@ -764,9 +767,14 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                         for (int k = 0; k < 4; ++k) {
                             float x = v[k];
                             if (CLIP && p.l_max > 0.0f) x = fminf(fmaxf(x, -p.l_max), p.l_max);
+                            if (SC) {
+                                x *= LLR_SCALE;
+                                far |= !(x * (1.0f / LLR_SCALE) == v[k]) || !(fabsf(x) < SCALED_LLR_LIMIT);
+                            }
                             L.st(4 * qd + k, x);
                         }
                     }
+                    if (SC && far) p.tally[T_OUT_OF_RANGE] = 1ull;
                 } else {
                     const uint64_t gf = p.first_frame + fid[f];
                     float ch_mu = p.mu, ch_sigma = p.sigma;
@@ -1091,7 +1099,7 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
             if (p.post_out) {
                 const SV L(sL, f, lstride);
                 float* dst = p.post_out + (size_t)fid[f] * N;
-                for (int i = tid; i < N; i += T) dst[i] = L.ld(i);
+                for (int i = tid; i < N; i += T) dst[i] = SC ? L.ld(i) * (1.0f / LLR_SCALE) : L.ld(i);
             }
         }
         need = done;

@@ -28,7 +28,7 @@ struct QcEntry {
 };
 // Which variants are built scaled: all but the plain shapes, which serve the channels outside its range.
 constexpr bool qc_scaled(int mode, int algo, bool clip, bool ext) {
-    return !ext && !clip && mode != 2 /* STORE_FP16 */ && (algo == 0 /* ALGO_AMIN */ || algo == 3 /* ALGO_CIRC */);
+    return !clip && mode != 2 /* STORE_FP16 */ && (algo == 0 /* ALGO_AMIN */ || (algo == 3 /* ALGO_CIRC */ && !ext));
 }
 
 struct QcTable {

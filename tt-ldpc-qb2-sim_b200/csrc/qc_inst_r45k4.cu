@@ -83,6 +83,8 @@ static const QcEntry qc_r45k4[] = {
     // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
     LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 6),
     LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 6),
+    // fp32 caller-supplied LLRs at LLR_SCALE (the unscaled counterpart is the larger cap)
+    LDPC_QC_ENTRY_GR(128, 18, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 5),
 };
 LDPC_QC_REGISTER(qc_r45k4)
 
@@ -101,6 +103,7 @@ static const QcDefault qc_r45k4_default[] = {
     {128, 18, STORE_FP32, ALGO_WROW, 0, 1, 1, 8, 1},
     {128, 18, STORE_BF16, -1, 300, 1, 1, 6, 7},
     {128, 18, STORE_FP16, -1, 300, 1, 1, 6, 7},
+    {128, 18, STORE_FP32, -1, 0, 1, 1, 5, 7},  // (caller-supplied LLRs only)
     {128, 18, STORE_FP32, -1, 0, 1, 1, 6, 7},
 };
 LDPC_QC_DEFAULTS(qc_r45k4_default)
