@@ -108,3 +108,37 @@ def test_workspace_is_no_larger_than_the_checkpoints_asked_for(gpu, K, rate):
                 for n in (0, 1, 3, 500, 4096):
                     got = capi._check(int(dec._lib.ldpc_wdec_workspace_bytes(dec._h, C.byref(cfg), n)))
                     assert got <= 4 * n * (-(-T // every) * (N + E) + (every + 2) * E), (T, every, n)
+
+
+@pytest.mark.parametrize("K,rate,T,every", [(1024, "1/2", 64, 8), (1024, "4/5", 45, 6)])
+def test_backward_can_be_repeated_over_several_segments(gpu, K, rate, T, every):
+    """Several segments before the kept iterations, two backward passes (the second runs the kept iterations
+    again from the last segment's state), against a plan that keeps every iteration: the same operations,
+    so the same bits, but for the order in which the CTAs add their parameter sums.  (Plain PyTorch breaks
+    ties in min and max its own way, which some forty iterations at 1.5 dB amplify to any size.)"""
+    code = ar4ja.make_code(K, rate)
+    llr, a, b = _inputs(code, 3, T, code.n_classes, 9)
+    gpost = torch.randn(T, 3, code.N, generator=torch.Generator().manual_seed(4)).to(DEV) / T
+    with capi.Decoder.from_code(code, 0) as dec:  # (through the C entries: WeightedFn frees its workspace)
+        lib = dec._lib
+        s = torch.cuda.current_stream().cuda_stream or None
+
+        def passes(every, n):
+            cfg = weighted.make_config(code, T, every)
+            nbytes = capi._check(int(lib.ldpc_wdec_workspace_bytes(dec._h, C.byref(cfg), 3)))
+            ws, post = torch.empty(nbytes, dtype=torch.uint8, device=DEV), torch.empty(T, 3, code.N, device=DEV)
+            capi._check(lib.ldpc_wdec_forward(dec._h, C.byref(cfg), llr.data_ptr(), 3, a.data_ptr(), b.data_ptr(),
+                                              post.data_ptr(), ws.data_ptr(), s))
+            for _ in range(n):
+                ga, gb, gx = torch.empty_like(a), torch.empty_like(b), torch.empty_like(llr)
+                capi._check(lib.ldpc_wdec_backward(dec._h, C.byref(cfg), 3, a.data_ptr(), b.data_ptr(),
+                                                   gpost.data_ptr(), ga.data_ptr(), gb.data_ptr(), gx.data_ptr(),
+                                                   ws.data_ptr(), s))
+                yield post, gx, ga, gb
+
+        ref, rx, ra, rb = next(passes(1, 1))
+        for post, gx, ga, gb in passes(every, 2):
+            assert torch.equal(post.view(torch.int32), ref.view(torch.int32))
+            assert torch.equal(gx.view(torch.int32), rx.view(torch.int32))
+            _close(ga, ra)
+            _close(gb, rb)

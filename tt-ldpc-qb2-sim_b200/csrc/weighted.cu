@@ -426,8 +426,8 @@ __host__ __device__ constexpr int wpad(int n) {
     return (n + (int)(16 / sizeof(Real)) - 1) & ~((int)(16 / sizeof(Real)) - 1);
 }
 
-// State i of frame b, at the start of a segment (iteration i * keep, or the first kept one for the last
-// i): L [N], then for i > 0 the messages (none before the first iteration).
+// State i of frame b, at the start of a segment (iteration i * keep): L [N], then for i > 0 the messages (none
+// before the first iteration).
 template <typename Real, int Z, int D>
 __device__ __forceinline__ Real* wckpt(const WParams& p, int i, int b) {
     const size_t n = p.n_frames, N = p.n_vars, S = N + 2 * (size_t)wedge_pairs(Z, D);
@@ -439,15 +439,16 @@ __device__ __forceinline__ Real* wckpt(const WParams& p, int i, int b) {
 // need no synchronisation.  L lives in shared memory, a barrier after every layer.
 //
 // The state kept for the backward pass: the q of every row of the last `keep` iterations (stash), and
-// when those are not all, the decoder's state at the iterations 0, keep, 2 keep, .. before them and at
-// the first of them (ckpt).  The messages of the frame being decoded sit in the stash's last iteration,
-// which is written only when they are no longer needed.
+// when those are not all, the decoder's state at the iterations 0, keep, 2 keep, .. before them (ckpt).
+// The messages of the frame being decoded sit in the stash's last iteration, which is written only when
+// they are no longer needed.  (A state at the first kept iteration as well, for repeated backward passes
+// only, took the room of a kept iteration's rows and cost 3 % here, 5 % of the backward kernel.)
 //
 // Bound by instruction issue (76 % of the slots, 42 lane instructions per edge and iteration at degree 6;
 // 2.9 TB/s of posteriors and stash written).  The layers of one degree share one body in a loop, so a kernel
 // is a few thousand instructions and its warps do not miss the instruction cache; a row's messages are
 // read and written as pairs and loaded a layer ahead.  r1/2 K=1024, 4096 frames, 20 iterations (B200,
-// 1965 MHz): 0.915 ms, 1.18 ms with the twelve layers unrolled and one word per message.
+// 1965 MHz): 0.89 ms, 1.18 ms with the twelve layers unrolled and one word per message.
 template <typename Real, int Z, int D>
 __global__ void __launch_bounds__(Z) wfwd_kernel(const __grid_constant__ WParams p) {
     using W2 = typename WPair<Real>::T;
@@ -470,8 +471,8 @@ __global__ void __launch_bounds__(Z) wfwd_kernel(const __grid_constant__ WParams
         W2 rr[(D + 1) / 2] = {};
         for (int t = 0; t < T; ++t) {
             wfill<Real, Z, D>(p, sw, cls, t, tid);
-            if (t < R ? t % K == 0 : R > 0 && t == R) {  // each thread stores its own variables and messages
-                Real* ck = wckpt<Real, Z, D>(p, (t + K - 1) / K, b);
+            if (t < R && t % K == 0) {  // each thread stores its own variables and messages
+                Real* ck = wckpt<Real, Z, D>(p, t / K, b);
                 for (int i = tid; i < N; i += Z) ck[i] = L[i];
                 if (t)
                     for (int i = tid; i < EP; i += Z) reinterpret_cast<W2*>(ck + N)[i] = r[i];
@@ -541,7 +542,7 @@ __device__ __forceinline__ void wbwd_iteration(const WParams& p, Real* X, typena
 // forward again from its state (stashing every layer's q in the frame's stash, whose kept iterations
 // are done with) and walked back.  The adjoint of the posteriors waits in global memory meanwhile.  A
 // second backward pass of the same forward pass finds the frame's stash used and runs its kept
-// iterations again as well.
+// iterations again as well, from the last state before them.
 //
 // Bound by instruction issue (64 % of the slots at 17 resident warps; about 75 lane instructions per edge
 // and iteration walked back, half of them on the half-rate ALU pipe, plus the forward's for those run
@@ -550,7 +551,7 @@ __device__ __forceinline__ void wbwd_iteration(const WParams& p, Real* X, typena
 // parameter gradients halved across the warp (wsum: 13 exchanges per degree-6 row instead of 60) and
 // kept per edge slot until the iteration ends, CTAs that stay for many frames (one global atomic per
 // CTA and parameter), and no second run of the kept iterations.  ms of the kernel, 20 iterations, every 5:
-// r1/2 K=1024, 4096 frames 7.47 -> 2.61; r4/5 K=4096, 512 frames, one class per row 5.37 -> 1.09.
+// r1/2 K=1024, 4096 frames 7.47 -> 2.47; r4/5 K=4096, 512 frames, one class per row 5.37 -> 1.02.
 template <typename Real, int Z, int D, int B>
 __global__ void __launch_bounds__(Z, B) wbwd_kernel(const __grid_constant__ WParams p) {
     using W2 = typename WPair<Real>::T;
@@ -580,20 +581,23 @@ __global__ void __launch_bounds__(Z, B) wbwd_kernel(const __grid_constant__ WPar
         for (int seg = n_seg; seg >= 0; --seg) {
             const int t0 = seg < n_seg ? seg * K : R, t1 = seg < n_seg ? min(R, t0 + K) : T;
             if (seg < n_seg || used) {
-                const Real* ck = wckpt<Real, Z, D>(p, seg, b);
+                // from the segment's own state, the kept part's again from the last one before it
+                const int ts = seg < n_seg ? t0 : (n_seg - 1) * K;
+                const Real* ck = wckpt<Real, Z, D>(p, ts / K, b);
                 for (int i = tid; i < N; i += Z) {  // each thread's own variables
                     save[i] = X[i];
                     X[i] = ck[i];
                 }
                 if (tid == 0) p.used[b] = 1;
-                const W2* r_in = t0 ? reinterpret_cast<const W2*>(ck + N) : nullptr;
+                const W2* r_in = ts ? reinterpret_cast<const W2*>(ck + N) : nullptr;
                 W2 rr[(D + 1) / 2] = {};
                 if (r_in) wload<Real, Z, D>(r_in, 0, tid, rr);
-                for (int t = t0; t < t1; ++t) {
+                for (int t = ts; t < t1; ++t) {
                     wfill<Real, Z, D>(p, sw, cls, t, tid);
                     __syncthreads();
                     wfwd_iteration<Real, Z, D, D <= 6 ? 2 : 1>(p, X, r_in, t < t1 - 1 ? r : nullptr,
-                                                               stash + (size_t)(t - t0) * EP, sw, tid, rr);
+                                                               t >= t0 ? stash + (size_t)(t - t0) * EP : nullptr, sw,
+                                                               tid, rr);
                     r_in = r;
                 }
                 for (int i = tid; i < N; i += Z) X[i] = save[i];
@@ -647,7 +651,7 @@ size_t weighted_plan(WParams* p, int Z, int D, int ckpt_every, int n_sm, size_t 
         const size_t R = T - K, seg = (R + K - 1) / K;
         p->keep = K;
         p->off_ckpt = n * (size_t)K * EP2;
-        p->off_gr = p->off_ckpt + (R ? n * (N + seg * (N + EP2)) : 0);
+        p->off_gr = p->off_ckpt + (R ? n * (N + (seg - 1) * (N + EP2)) : 0);
         p->off_save = p->off_gr + p->n_slots * EP2;
         p->off_used = p->off_save + p->n_slots * N;
         return (p->off_used + n) * rb + W_ALIGN;
