@@ -108,11 +108,12 @@ static const QcEntry qc_r12k1[] = {
 };
 LDPC_QC_REGISTER(qc_r12k1)
 
-// Default shapes (us of the kernel at 1 / 440 / 1500 / 100000 frames, 2.04 dB, Approximate-Min*).  Below about
-// 2500 frames a kernel waits for its slowest frame and fewer registers per thread do not help; above,
-// resident warps and instructions decide.  (Layout 6 cap 5 at 1 / 440 / 1500 frames, 2.0 dB, all other kernels timed
-// again beside it: bf16 21.5 / 48.1 / 105.5, cap 8 25.6 / 54.1 / 109.5, layout 0 cap 5 22.5 / 50.2 / 113.6; fp16 20.5 / 48.2 /
-// 102.4, layout 0 cap 5 21.5 / 52.2 / 117.8.)
+// Default shapes (us of the kernel at 1 / 440 / 1500 / 100000 frames, 2.04 dB, Approximate-Min*).  Few frames
+// wait for the slowest of them, where fewer registers per thread do not help; with many, resident warps and
+// instructions decide.  Layout 6 cap 5 is ahead at both ends since its min* step is one instruction shorter
+// (amin_step_scaled): bf16 at 1 / 440 / 1500 / 5000 / 100000 frames 21.5 / 43.2 / 98 / 276 / 4982 against cap 8 25.6 / 54.1 /
+// 109.5 / 284 / 5067, caller-supplied LLRs (8000 frames) 429 against 445; fp16 (20.5 / 48.2 / 102.4) / 285 / 5102 against
+// layout 2 cap 6 289 / 5173.  The figures below were taken before that, of one run each.
 //   bf16: layout 0 cap 5 25.0 / 47.5 / 110.8 / 5831, layout 6 cap 8 27.6 / 50.2 / 108.6 / 5269, layout 2 cap 8 - / 53.5 / 109.0 / 5335,
 //         (1,1,0,0) 26.9 / 52.2 / 119.0 / 6268
 //   fp16: layout 0 cap 5 23.5 / 46.3 / 110.8 / 5780, layout 2 cap 6 26.8 / 47.5 / 104.9 / 5171, layout 6 cap 6 24.9 / 45.4 / 104.8 /
@@ -126,13 +127,11 @@ static const QcDefault qc_r12k1_default[] = {
     {128, 6, STORE_FP32, ALGO_WAMIN, 1500, 1, 1, 0, 2},
     {128, 6, STORE_FP32, ALGO_WAMIN, 0, 1, 1, 0, 0},
     {128, 6, STORE_FP16, ALGO_WAMIN, 0, 1, 1, 5, 0},
-    {128, 6, STORE_BF16, -1, 2500, 1, 1, 8, 6},
     {128, 6, STORE_BF16, -1, 0, 1, 1, 5, 6},
     {128, 6, STORE_BF16, -1, 1500, 1, 1, 8, 6},
     {128, 6, STORE_BF16, -1, 1500, 1, 1, 8, 2},
     {128, 6, STORE_BF16, -1, 1500, 1, 1, 0, 2},
     {128, 6, STORE_BF16, -1, 0, 1, 1, 5, 0},
-    {128, 6, STORE_FP16, -1, 2500, 1, 1, 6, 2},
     {128, 6, STORE_FP16, -1, 0, 1, 1, 5, 6},
     {128, 6, STORE_FP16, -1, 1500, 1, 1, 6, 2},
     {128, 6, STORE_FP16, -1, 1500, 1, 1, 6, 6},
