@@ -92,3 +92,16 @@ def test_handles_on_several_threads(gpu):
     [t.start() for t in ts]
     [t.join() for t in ts]
     assert not bad
+
+
+def test_one_copy_up_to_250_kilobytes(gpu):
+    """250 KiB of fp32 LLRs is 31 frames of 2048; of posteriors and counts 24 frames of 2560."""
+    code = ar4ja.make_code(1024, "1/2")
+    llr = _frames(code, 64, 6)
+    with capi.Decoder.from_code(code) as d:
+        want = d.decode_llr(llr, max_iter=40, storage="bf16")
+        for n in (23, 24, 25, 30, 31, 32, 33):
+            for post in (True, False):
+                got = d.decode_llr(llr[:n], max_iter=40, storage="bf16", want_post=post)
+                assert all(np.array_equal(a, b[:n]) for a, b in zip(got[1:4], want[1:4]))
+                assert not post or np.array_equal(got[0].view(np.uint32), want[0][:n].view(np.uint32))

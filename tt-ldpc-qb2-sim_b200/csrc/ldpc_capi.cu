@@ -111,13 +111,17 @@ struct ldpc_handle {
     static constexpr int hist_bins = 1024;
     static constexpr size_t kCounterBytes = 64 + hist_bins * 8 + 4 * SNR_BINS * 8 + TALLY_WORDS * 8;
     static constexpr size_t kTallyOff = kCounterBytes - TALLY_WORDS * 8;
-    // LLRs (as fp32) and outputs of a small call, at most this much each; then the same LLRs as bf16
-    static constexpr size_t kSmallBytes = 1u << 20;
+    // LLRs (as fp32) and outputs of a small call, at most this much each; then the same LLRs as bf16.  So large that
+    // one frame of any code fits, and that the pinned buffer stays at 512 KB, up to which pinning takes some
+    // microseconds (a share of memory the runtime has pinned already) and above which 1 to 5 ms a handle.
+    static constexpr size_t kSmallBytes = 250u << 10;
     static constexpr size_t kSmallLlr = (kCounterBytes + kSmallBytes + 255) / 256 * 256;
     static constexpr size_t kSmallLlr16 = kSmallLlr + kSmallBytes;
     static constexpr size_t kIoBytes = kSmallLlr16 + kSmallBytes / 2;
     unsigned char* h_small = nullptr;  // pinned: the tally, a small call's outputs, its LLRs
     static constexpr size_t kSmallHostLlr = (TALLY_WORDS * 8 + kSmallBytes + 255) / 256 * 256;
+    static constexpr size_t kSmallHost = kSmallHostLlr + kSmallBytes;
+    static_assert(kSmallHost <= 512u << 10, "");
     float* d_llr = nullptr;
     size_t llr_cap = 0;
     float* d_post = nullptr;
@@ -309,7 +313,7 @@ extern "C" int ldpc_create(const ldpc_matrix* m, int device, ldpc_handle** out) 
         cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
         return bail(fail(LDPC_EIO, "stream/event creation failed"));
     if (cudaMalloc(&h->d_io, ldpc_handle::kIoBytes) != cudaSuccess ||
-        cudaMallocHost(&h->h_small, ldpc_handle::kSmallHostLlr + ldpc_handle::kSmallBytes) != cudaSuccess)
+        cudaMallocHost(&h->h_small, ldpc_handle::kSmallHost) != cudaSuccess)
         return bail(fail(LDPC_ENOMEM, "device allocation failed"));
     h->h_tally = reinterpret_cast<unsigned long long*>(h->h_small);
     h->d_work = reinterpret_cast<unsigned int*>(h->d_io);
@@ -1175,15 +1179,22 @@ static int host_outputs(ldpc_handle* h, size_t nb, bool plain, float* post, int3
     } else if (post) {
         CU(cudaMemcpyAsync(post, h->d_post, nb * h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     }
-    // the per-frame counts: one copy into the pinned buffer where they fit, else one per array
-    if (plain && 3 * nb * sizeof(int32_t) <= ldpc_handle::kSmallBytes) {
-        unsigned char* buf = h->h_small + TALLY_WORDS * 8;
-        CU(cudaMemcpyAsync(buf, d_it, 3 * nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-        if ((rc = read_tally(h, out))) return rc;
-        const int32_t* o = reinterpret_cast<const int32_t*>(buf);
-        if (iters) memcpy(iters, o, nb * sizeof(int32_t));
-        if (synd_fail) memcpy(synd_fail, o + nb, nb * sizeof(int32_t));
-        if (bit_errors) memcpy(bit_errors, o + 2 * nb, nb * sizeof(int32_t));
+    // the per-frame counts: through the pinned buffer where it takes a few copies, else one copy per array
+    constexpr size_t kPiece = (ldpc_handle::kSmallHost - TALLY_WORDS * 8) / sizeof(int32_t);
+    if (plain && 3 * nb <= 4 * kPiece) {
+        const int32_t* o = reinterpret_cast<const int32_t*>(h->h_small + TALLY_WORDS * 8);
+        int32_t* dst[3] = {iters, synd_fail, bit_errors};
+        for (size_t a = 0; a < 3 * nb; a += kPiece) {
+            const size_t b = std::min(a + kPiece, 3 * nb);
+            CU(cudaMemcpyAsync(h->h_small + TALLY_WORDS * 8, d_it + a, (b - a) * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                               h->stream));
+            if (b < 3 * nb) CU(cudaStreamSynchronize(h->stream));
+            else if ((rc = read_tally(h, out))) return rc;
+            for (size_t k = 0; k < 3; ++k) {
+                const size_t lo = std::max(a, k * nb), hi = std::min(b, (k + 1) * nb);
+                if (dst[k] && lo < hi) memcpy(dst[k] + (lo - k * nb), o + (lo - a), (hi - lo) * sizeof(int32_t));
+            }
+        }
         return 0;
     }
     if (iters) CU(cudaMemcpyAsync(iters, d_it, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
