@@ -500,8 +500,9 @@ int launch_general(GeneralCode* g, const ldpc_run_params* p, bool ext, uint32_t 
 // A matrix with the quasi-cyclic structure runs on the QC kernel (run_static_qc): its messages stay in
 // registers or take one slot per CTA, it needs no row schedule, and a frame has a whole CTA instead of one
 // warp.  LLRs in range run on the scaled kernels; all else on the variants with the clips compiled in, whatever
-// the clips (with infinite caps they change only a NaN posterior, to -inf, as the general kernel does).  4001 frames r1/2 K=1024 bf16 2.0 dB with
-// posteriors: 3.00 ms on the general kernel (1.41 of them its schedule), 0.29.
+// the clips (with infinite caps they change only a NaN posterior, to -inf, as the general kernel does).  4001
+// frames r1/2 K=1024 bf16 2.0 dB with posteriors: 3.00 ms on the general kernel (1.41 of them the schedule of
+// that time), 0.27.
 //
 // Scratch layout of the general kernel (LDPC_STATIC_SCRATCH_BYTES, 256-byte aligned regions):
 //   [0, 256)           frame-claim counter (u32) and tallies (TALLY_WORDS x u64)
@@ -693,8 +694,8 @@ static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const f
         cudaGetLastError();
         return LDPC_ENOTSUP;
     }
-    // the default shape (unscaled: its variant with clips); a shape with messages in global memory only if the scratch holds a slot for every
-    // resident CTA, or if there is no other
+    // the default shape (unscaled: its variant with clips); a shape with messages in global memory only if the
+    // scratch holds a slot for every resident CTA, or if there is no other
     const void* fn = nullptr;
     int sh[4];
     size_t smem = 0;
