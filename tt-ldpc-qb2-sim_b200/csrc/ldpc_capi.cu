@@ -1135,7 +1135,8 @@ static int decode_small(ldpc_handle* h, const ldpc_run_params* p, const void* ll
 }
 
 // Device -> host copy into a pageable array through the pinned ring: while the host copies one piece out of its
-// slot (threads share the work, and the page faults of a fresh array), the next piece travels.
+// slot (threads share the work, and the page faults of a fresh array), the next piece travels.  Only where the ring is
+// there already, for pageable LLRs: pinning its 96 MB takes some 50 ms, the copy of 41 MB by the driver 0.4 ms more.
 static int unstage_d2h(ldpc_handle* h, char* dst, const char* src, size_t bytes) {
     int rc;
     if ((rc = stage_alloc(h))) return rc;
@@ -1172,7 +1173,7 @@ static int host_outputs(ldpc_handle* h, size_t nb, bool plain, float* post, int3
     if (!nb) return read_tally(h, out);
     int32_t *d_it = h->d_frame_out, *d_sf = d_it + nb, *d_be = d_sf + nb;
     bool ring = false;
-    if (post && host_memory(post, &ring) && ring) {
+    if (post && host_memory(post, &ring) && ring && h->stage[ldpc_handle::kStageSlots - 1]) {
         if ((rc = unstage_d2h(h, reinterpret_cast<char*>(post), reinterpret_cast<const char*>(h->d_post),
                               nb * h->N * sizeof(float))))
             return rc;
