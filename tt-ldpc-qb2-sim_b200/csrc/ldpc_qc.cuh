@@ -638,6 +638,15 @@ __device__ __forceinline__ int qc_blk(const QcParams& p, int l, int e) {
     if constexpr (FIX >= 0) return kQcFixedDev[FIX].blk_off[l][e];
     else return p.blk_off[l][e];
 }
+// Whether a caller's channel LLR v may be decoded as x = v LLR_SCALE: below 2^20 (and not NaN), and x exact as it is
+// stored.  A bf16 subnormal has fewer bits than the bf16 of v, so with bf16 storage x is zero or normal (|v| >=
+// 2^-76); every value computed from such LLRs is then a multiple of 2^-83, as bf16 at LLR_SCALE a multiple of its
+// smallest subnormal.  In fp32 the product is exact down to the last bit of its subnormals.
+template <int MODE> __device__ __forceinline__ bool llr_scales(float v, float x) {
+    const bool exact = MODE == STORE_BF16 ? v == 0.0f || fabsf(x) >= 1.17549435e-38f : x * (1.0f / LLR_SCALE) == v;
+    return exact && fabsf(x) < SCALED_LLR_LIMIT;
+}
+
 template <int FIX>
 __device__ __forceinline__ int qc_shift(const QcParams& p, int l, int e) {
     if constexpr (FIX >= 0) return kQcFixedDev[FIX].shift[l][e];
@@ -655,7 +664,7 @@ __device__ __forceinline__ int qc_shift(const QcParams& p, int l, int e) {
 // only for a matrix whose descriptors are those).
 // SC: the frames are decoded at LLR_SCALE (Approximate-Min*, or the simulation of the circulant engine's decoder;
 // fp32 or bf16 storage, no clips): the same values but for the scale, one instruction less per min* step.  A
-// caller's LLR that does not scale exactly or is 2^20 or more (or NaN) is reported in the tally.
+// caller's LLR out of range (llr_scales) is reported in the tally.
 // ROLL (layout 7, global messages only): the eight degree-D layers run as one loop that is not
 // unrolled, each row's descriptors read from the kernel parameters by layer index.  The unrolled
 // body of a degree-18 code is tens of KB of instructions; with one-warp CTAs whose warps are
@@ -769,7 +778,7 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                             if (CLIP && p.l_max > 0.0f) x = fminf(fmaxf(x, -p.l_max), p.l_max);
                             if (SC) {
                                 x *= LLR_SCALE;
-                                far |= !(x * (1.0f / LLR_SCALE) == v[k]) || !(fabsf(x) < SCALED_LLR_LIMIT);
+                                far |= !llr_scales<MODE>(v[k], x);
                             }
                             L.st(4 * qd + k, x);
                         }
