@@ -114,7 +114,13 @@ __global__ void __launch_bounds__(32, STEP_MIN_CTAS) general_step_kernel(const _
     uint32_t* rs = reinterpret_cast<uint32_t*>(p.r_base) + (size_t)blockIdx.x * ((size_t)S * W * 32) + lane;
     const float inf = __int_as_float(0x7f800000);
     const float r_cap = CLIP && p.r_max > 0.0f ? p.r_max : inf;
+    // the warp's tallies, kept by lane 0: SC in shared memory, as the QC kernel's
+    __shared__ unsigned long long s_tally[SC ? TALLY_WORDS : 1];
     unsigned long long t_frames = 0, t_be = 0, t_fe = 0, t_it = 0, t_unc = 0, t_max = 0, t_be2 = 0;
+    if (SC && lane == 0)
+        for (int i = 0; i < TALLY_WORDS; ++i) s_tally[i] = 0;
+    const int pad = N * (int)sizeof(LE);  // the dummy slot's column entry
+    float hi = 0.0f;                      // SC: 1 or more once a magnitude of this lane's rows has been 1
 
     for (;;) {
         uint32_t fid = 0;
@@ -187,10 +193,10 @@ __global__ void __launch_bounds__(32, STEP_MIN_CTAS) general_step_kernel(const _
             else mn[0].zero();
             if (low) {
                 row_update<DL, MODE, ALGO, CLIP, 1, MSG, true, true, SC>(reinterpret_cast<const int(&)[DL]>(c), L, 0, m,
-                                                                     r_cap, inf);
+                                                                         r_cap, inf, hi, nullptr, pad);
                 msg_store<DT, MODE, step_words<MODE>(DL)>(rs, s, m[0]);
             } else {
-                row_update<DT, MODE, ALGO, CLIP, 1, MSG, true, true, SC>(c, L, 0, m, r_cap, inf);
+                row_update<DT, MODE, ALGO, CLIP, 1, MSG, true, true, SC>(c, L, 0, m, r_cap, inf, hi, nullptr, pad);
                 msg_store<DT, MODE>(rs, s, m[0]);
             }
             __syncwarp();
@@ -226,13 +232,6 @@ __global__ void __launch_bounds__(32, STEP_MIN_CTAS) general_step_kernel(const _
                 }
             }
         }
-        if constexpr (SC) {
-            if (it >= SCALED_CHECK_FROM) {
-                bool far = false;
-                for (int i = lane; i < N; i += 32) far |= !(fabsf(LT::ld(L, i)) < SCALED_LIMIT);
-                if (far) p.tally[T_OUT_OF_RANGE] = 1ull;
-            }
-        }
         // tally
         uint32_t be = 0;
         for (int i = lane; i < p.n_tx; i += 32) be += LT::sign(L, i);
@@ -250,13 +249,23 @@ __global__ void __launch_bounds__(32, STEP_MIN_CTAS) general_step_kernel(const _
             sfail = __reduce_add_sync(0xFFFFFFFFu, sfail);
         }
         if (lane == 0) {
-            t_frames += 1;
-            t_be += be;
-            t_be2 += (unsigned long long)be * be;
-            t_fe += be > 0;
-            t_it += (unsigned)it;
-            t_unc += sfail != 0;
-            t_max = max(t_max, (unsigned long long)it);
+            if constexpr (SC) {
+                s_tally[T_FRAMES] += 1;
+                s_tally[T_BIT_ERR] += be;
+                s_tally[T_BIT_ERR_SQ] += (unsigned long long)be * be;
+                s_tally[T_FRAME_ERR] += be > 0;
+                s_tally[T_ITER_SUM] += (unsigned)it;
+                s_tally[T_UNCONVERGED] += sfail != 0;
+                s_tally[T_MAX_ITER] = max(s_tally[T_MAX_ITER], (unsigned long long)it);
+            } else {
+                t_frames += 1;
+                t_be += be;
+                t_be2 += (unsigned long long)be * be;
+                t_fe += be > 0;
+                t_it += (unsigned)it;
+                t_unc += sfail != 0;
+                t_max = max(t_max, (unsigned long long)it);
+            }
             if (p.hist) atomicAdd(&p.hist[min(it, p.hist_bins - 1)], 1ull);
             if (per_frame_snr && p.snr_bins) {
                 atomicAdd(&p.snr_bins[snr_bin], 1ull);
@@ -273,6 +282,17 @@ __global__ void __launch_bounds__(32, STEP_MIN_CTAS) general_step_kernel(const _
             for (int i = lane; i < N; i += 32) dst[i] = LT::ld(L, __ldg(slot + i));
         }
         __syncwarp();
+    }
+    if constexpr (SC) {
+        if (hi >= 1.0f) p.tally[T_OUT_OF_RANGE] = 1ull;
+        if (lane != 0) return;
+        t_frames = s_tally[T_FRAMES];
+        t_be = s_tally[T_BIT_ERR];
+        t_be2 = s_tally[T_BIT_ERR_SQ];
+        t_fe = s_tally[T_FRAME_ERR];
+        t_it = s_tally[T_ITER_SUM];
+        t_unc = s_tally[T_UNCONVERGED];
+        t_max = s_tally[T_MAX_ITER];
     }
     if (lane == 0 && t_frames) {
         atomicAdd(&p.tally[T_FRAMES], t_frames);

@@ -67,8 +67,8 @@ static const QcEntry* find_qc(const QcKey& k, bool scaled) {
 }
 
 // Whether the scaled kernels may decode a simulated channel: LLR mean and deviation between 2^-10 and 2^12 (or 0),
-// i.e. an Eb/N0 between about -30 and 30 dB, and at most 10000 iterations; values then stay far inside the
-// range LLR_SCALE leaves, and the kernel checks long frames all the same.
+// i.e. an Eb/N0 between about -30 and 30 dB, and at most 10000 iterations; no channel value is then too small to
+// scale exactly, and the kernels watch for magnitudes that grow past what LLR_SCALE leaves.
 // Caller-supplied LLRs (ext) are checked by the kernel.
 static bool qc_scaled_ok(const ldpc_run_params* p, bool ext) {
     if (ext) return p->max_iter <= 10000;

@@ -115,11 +115,16 @@ __device__ __forceinline__ float amin_step_fma(float m, float a) {
     return fmaxf(__fmaf_rn(-c, f2, cur), 0.0f);
 }
 
-// The same step on values scaled by 2^-50, so that a saturating result clamps at 0 and never at 1 for values below
+// The same step on values scaled by 2^-50, so that a saturating result clamps at 0 and not at 1 for values below
 // 2^50: one instruction less (the clamp is the last multiply-add's).  Scaling by a power of two commutes with every
-// rounding here, so the values are exactly 2^-50 times amin_step_fma's: nothing a decoder of in-range channel
-// values (qc_scaled_ok) computes is large enough to saturate (posteriors stay below 300; 2^50 is 1e15) or small
-// enough to lose bits (channel values are multiples of 2^-93; scaled, of 2^-143, which a denormal holds).
+// rounding here, so the values are exactly 2^-50 times amin_step_fma's, as long as
+//  - no magnitude reaches 2^50, where the step saturates.  No bound follows from the channel: a row's minimum is
+//    capped at 9999, but the magnitude sent to the edge that counts as its minimum is not, and on a matrix whose
+//    columns are each that edge in several rows the values double every iteration.  So every row's magnitude is
+//    looked at (`hi` of row_update, one maximum a row; on the AR4JA codes posteriors stay below 300 at any SNR a
+//    simulation runs at), and one that has saturated makes the host decode the call again on the unscaled kernels;
+//  - nothing is small enough to lose bits: a simulated channel value (qc_scaled_ok) is 0 or at least 2^-57, a
+//    multiple of 2^-93, scaled of 2^-143, which a denormal holds; caller-supplied LLRs are checked (llr_scales).
 // r1/2 K=1024 fp32 26.3 -> 27.6, bf16 23.5 -> 24.6 M frames/s at 2.5 dB; K=16384 +3 to +5 %.
 constexpr float LLR_SCALE = 8.8817841970012523e-16f;  // 2^-50
 __device__ __forceinline__ float amin_step_scaled(float m, float a) {
@@ -132,10 +137,6 @@ __device__ __forceinline__ float amin_step_scaled(float m, float a) {
     const float c = diff < 0.5f * S ? c1 : c2;
     return __saturatef(__fmaf_rn(-c, f2, cur));
 }
-// A scaled frame's magnitudes are checked where they could have grown: frames of at least this many iterations,
-// against 2^40.  One beyond it makes the host decode the call again on the unscaled kernels.
-constexpr int SCALED_CHECK_FROM = 40;
-constexpr float SCALED_LIMIT = 9.765625e-4f;            // 2^40 scaled
 constexpr float SCALED_LLR_LIMIT = 9.3132257461547852e-10f;  // 2^20 scaled: caller-supplied channel LLRs
 
 // The circulant engine's min* (tests/test_circulant_dma_stepper.cpp:39-54 and

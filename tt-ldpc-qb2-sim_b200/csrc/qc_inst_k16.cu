@@ -37,7 +37,7 @@ static const QcEntry qc_k16[] = {
     LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_BF16, ALGO_AMIN, false, false, 2, 2),
     LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_FP16, ALGO_AMIN, false, false, 2, 2),
     // the same for caller-supplied LLRs
-    LDPC_QC_ENTRY_GF(1024, 10, 2, 1, STORE_BF16, ALGO_AMIN, false, true, 0, 1),
+    LDPC_QC_ENTRY_GF(1024, 10, 2, 1, STORE_BF16, ALGO_AMIN, false, true, 2, 1),
     LDPC_QC_ENTRY_GF(1024, 10, 2, 1, STORE_FP16, ALGO_AMIN, false, true, 2, 1),
     LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_BF16, ALGO_AMIN, false, true, 2, 2),
     LDPC_QC_ENTRY_GF(512, 18, 1, 1, STORE_FP16, ALGO_AMIN, false, true, 2, 2),
@@ -75,11 +75,14 @@ LDPC_QC_REGISTER(qc_k16)
 //        4672 against 115.0 / 133.3 / 369.0 / 4800
 //   r4/5 bf16 cap 2 90.4 / 108.7 / 241.7 / 3026, uncapped 86.2 / 102.6 / 260.4 / 3372, parameters 88.2 / 106.5 / 272.5 / 3507;
 //        fp16 cap 2 92.4 / 110.9 / 243.9 / 3050 against 88.2 / 106.6 / 274.5 / 3522
+// Scaled kernels add up their rows' magnitudes (`hi` of row_update), which takes r2/3 bf16 without a cap past 64 registers, to
+// one CTA an SM: 3750 frames 2270 us before, 2598 since, cap 2 2285; caller-supplied LLRs, 500 frames, 367, 423, 378.
 // Min-sum and the clips have only these shapes: bf16 r1/2 192.7 / 192.9 / 455.0 and 207.0 / 209.0 / 526.6, r2/3 112.9 / 114.8 /
 // 282.9 and 121.0 / 139.5 / 344.4, r4/5 80.0 / 94.5 / 213.1 and 94.3 / 113.0 / 260.2 (the general kernel before).
 static const QcDefault qc_k16_default[] = {
     {2048, 6, STORE_BF16, -1, 0, 4, 1, 0, 5},
     {2048, 6, STORE_FP16, -1, 0, 4, 1, 0, 5},
+    {1024, 10, STORE_BF16, -1, 0, 2, 1, 2, 5},
     {1024, 10, STORE_BF16, -1, 0, 2, 1, 0, 5},
     {1024, 10, STORE_FP16, -1, 0, 2, 1, 2, 5},
     {512, 18, STORE_BF16, -1, 200, 1, 1, 2, 5},

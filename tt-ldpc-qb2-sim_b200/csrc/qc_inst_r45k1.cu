@@ -61,7 +61,7 @@ static const QcEntry qc_r45k1[] = {
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 16),
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 24),
     // fp32 caller-supplied LLRs at LLR_SCALE (the unscaled counterpart is the larger cap)
-    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 22),
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 20),
 };
 LDPC_QC_REGISTER(qc_r45k1)
 
@@ -73,7 +73,7 @@ LDPC_QC_REGISTER(qc_r45k1)
 static const QcDefault qc_r45k1_default[] = {
     {32, 18, STORE_BF16, -1, 0, 1, 1, 16, 7},
     {32, 18, STORE_FP16, -1, 0, 1, 1, 16, 7},
-    {32, 18, STORE_FP32, -1, 0, 1, 1, 22, 7},  // (caller-supplied LLRs only)
+    {32, 18, STORE_FP32, -1, 0, 1, 1, 20, 7},  // (caller-supplied LLRs only)
     {32, 18, STORE_FP32, -1, 0, 1, 1, 24, 7},
 };
 LDPC_QC_DEFAULTS(qc_r45k1_default)
