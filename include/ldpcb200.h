@@ -99,7 +99,8 @@ typedef struct {
     uint64_t max_iters;    /* largest iteration count of one frame */
     float kernel_ms;       /* device time of the decode kernel (CUDA events on the handle's stream;
                               for a large ldpc_decode_llr, from the first launch to the end of the
-                              last, waits for later chunks' LLR copies included) */
+                              last, waits for later chunks' LLR copies included), of every pass
+                              where frames are decoded again */
     float reserved1;
     uint64_t bit_errors_sq; /* sum over frames of (bit errors of the frame)^2: the frame-level variance
                                of the bit-error count, for confidence intervals on BER */
@@ -145,7 +146,9 @@ int ldpc_run_chunk(ldpc_handle* h, const ldpc_run_params* p, ldpc_tally* out);
  * decoding of the previous one).  Uses
  * p->max_iter, storage, algo and the clips (mu/sigma/seed ignored).  Outputs (each may be NULL):
  * post [n_frames][N] final L as stored (bf16/fp16 values widened to float), iters, synd_fail (rows
- * failing after decoding), bit_errors. */
+ * failing after decoding), bit_errors.  Frames with an LLR of 2^20 or more (known bits), infinite,
+ * not a number or below 2^-76 are decoded by kernels of their own, after the others: the same
+ * results, at the rate of the plain launch shape. */
 int ldpc_decode_llr(ldpc_handle* h, const ldpc_run_params* p, const float* llr, int64_t n_frames,
                     float* post, int32_t* iters, int32_t* synd_fail, int32_t* bit_errors,
                     ldpc_tally* out);
@@ -332,7 +335,7 @@ void ldpc_batch_destroy(ldpc_batch* b);
  * starts a code's CTAs as the CTAs launched before it retire); otherwise kernel i is limited to the
  * fraction share[i] / sum(share) of the GPU's CTA slots.
  * out[i] receives handle i's tallies (kernel_ms = the whole graph's device time), *graph_ms the
- * device time of the launch.  ldpc_snr_bins(handle i) then gives its per-Eb/N0 tallies. */
+ * device time of the launch (of both, where values too large for the first make it run again).  ldpc_snr_bins(handle i) then gives its per-Eb/N0 tallies. */
 int ldpc_batch_run(ldpc_batch* b, const ldpc_run_params* params, const float* share, ldpc_tally* out,
                    float* graph_ms);
 

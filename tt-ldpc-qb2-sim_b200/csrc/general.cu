@@ -675,10 +675,11 @@ constexpr uint64_t kStaticLaunchFrames = 1ull << 31;
 
 // The QC kernel on the static scratch: [0, 256) as for the general kernel, then the message slots of the
 // shapes that keep them in global memory.  LDPC_ENOTSUP (nothing launched): the matrix, the options or
-// the alignment of d_llr (the kernel reads four LLRs at a time) ask for the general kernel.
+// the alignment of d_llr (the kernel reads four LLRs at a time) ask for the general kernel.  left_out: only the frames
+// that the scaled pass before has left out.
 static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const float* d_llr, uint64_t n, float* d_post,
                          int32_t* d_iters, int32_t* d_synd, int32_t* d_be, ldpc_tally* out, unsigned char* base, int dev,
-                         cudaStream_t stream, std::string& err, bool scaled) {
+                         cudaStream_t stream, std::string& err, bool scaled, bool left_out = false) {
     const int N = h->n_vars, P = h->n_punct;
     QcStructure s = {};
     if (!n || (N - P) % 32 || reinterpret_cast<uintptr_t>(d_llr) % 16 ||
@@ -731,11 +732,12 @@ static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const f
     qp.l_max = p->l_max;
     qp.r_max = p->r_max;
     qp.l_post_max = p->l_post_max;
-    qp.work = reinterpret_cast<unsigned int*>(base);
+    qp.work = reinterpret_cast<unsigned int*>(base + (left_out ? 32 : 0));
+    qp.redo = left_out ? 1 : 0;
     qp.tally = reinterpret_cast<unsigned long long*>(base + 64);
     qp.hist_bins = 1;
     qp.r_base = base + 256;
-    cudaError_t e = cudaMemsetAsync(base, 0, 256, stream);
+    cudaError_t e = left_out ? cudaSuccess : cudaMemsetAsync(base, 0, 256, stream);
     for (uint64_t off = 0; e == cudaSuccess && off < n; off += kStaticLaunchFrames) {
         qp.n_frames = (uint32_t)std::min<uint64_t>(kStaticLaunchFrames, n - off);
         qp.llr_in = d_llr + off * (uint64_t)(N - P);
@@ -756,6 +758,8 @@ static int run_static_qc(const ldpc_matrix* h, const ldpc_run_params* p, const f
         return LDPC_EIO;
     }
     if (t[T_OUT_OF_RANGE]) return LDPC_ENOTSUP;  // scaled only: the caller decodes the frames again unscaled
+    if (scaled && t[T_LEFT_OUT])                 // the frames with LLRs out of range
+        return run_static_qc(h, p, d_llr, n, d_post, d_iters, d_synd, d_be, out, base, dev, stream, err, false, true);
     tally_out(t, out);
     return 0;
 }

@@ -121,7 +121,8 @@ struct ldpc_handle {
     unsigned char* h_small = nullptr;  // pinned: the tally, a small call's outputs, its LLRs
     static constexpr size_t kSmallHostLlr = (TALLY_WORDS * 8 + kSmallBytes + 255) / 256 * 256;
     static constexpr size_t kSmallHost = kSmallHostLlr + kSmallBytes;
-    static_assert(kSmallHost <= 512u << 10, "");
+    static_assert(kSmallHost + 4 <= 512u << 10, "");
+    uint32_t* left_flag = nullptr;  // behind them, set by the scaled kernels (QcParams)
     float* d_llr = nullptr;
     size_t llr_cap = 0;
     float* d_post = nullptr;
@@ -139,10 +140,11 @@ struct ldpc_handle {
     ldpc_circ_config circ{LDPC_CIRC_SFPU, LDPC_CIRC_STOP_GENIE, 0.9375f, 0};
     unsigned long long* h_tally = nullptr;  // the start of h_small
     int64_t launches = 0;
+    float ms_before = 0.0f;   // a call that decodes frames again: the time of its passes so far
     // ldpc_decode_llr: a copy stream and an event that let the decoding of one chunk of frames
     // overlap the host->device copy of the next (created on first use)
     cudaStream_t cstream = nullptr;
-    cudaEvent_t cev = nullptr;
+    cudaEvent_t cev[3] = {};  // of the last three chunks
     // ldpc_decode_llr_bf16: the caller's bf16 LLRs on the device before they are widened
     uint16_t* d_llr16 = nullptr;
     size_t llr16_cap = 0;
@@ -254,7 +256,8 @@ extern "C" void ldpc_destroy(ldpc_handle* h) {
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
-    if (h->cev) cudaEventDestroy(h->cev);
+    for (cudaEvent_t e : h->cev)
+        if (e) cudaEventDestroy(e);
     if (h->cstream) cudaStreamDestroy(h->cstream);
     cudaFree(h->d_llr16);
     for (int i = 0; i < ldpc_handle::kStageSlots; ++i) {
@@ -313,9 +316,10 @@ extern "C" int ldpc_create(const ldpc_matrix* m, int device, ldpc_handle** out) 
         cudaEventCreate(&h->ev0) != cudaSuccess || cudaEventCreate(&h->ev1) != cudaSuccess)
         return bail(fail(LDPC_EIO, "stream/event creation failed"));
     if (cudaMalloc(&h->d_io, ldpc_handle::kIoBytes) != cudaSuccess ||
-        cudaMallocHost(&h->h_small, ldpc_handle::kSmallHost) != cudaSuccess)
+        cudaMallocHost(&h->h_small, ldpc_handle::kSmallHost + 4) != cudaSuccess)
         return bail(fail(LDPC_ENOMEM, "device allocation failed"));
     h->h_tally = reinterpret_cast<unsigned long long*>(h->h_small);
+    h->left_flag = reinterpret_cast<uint32_t*>(h->h_small + ldpc_handle::kSmallHost);
     h->d_work = reinterpret_cast<unsigned int*>(h->d_io);
     h->d_hist = reinterpret_cast<unsigned long long*>(h->d_io + 64);
     h->d_snr = h->d_hist + h->hist_bins;
@@ -654,6 +658,9 @@ struct QcLaunch {
     int block = 0;
     size_t smem = 0;
     QcParams qp;
+    bool left_out = false;  // set before: for the frames the scaled kernel before has left out
+    bool scaled = false;    // the kernel decodes at LLR_SCALE
+    int frames_per_cta = 0;
 };
 
 static double code_rate(const ldpc_handle* h) { return (double)(h->N - h->M) / (double)(h->N - h->P); }
@@ -790,21 +797,40 @@ static int prepare_qc_shape(ldpc_handle* h, const ldpc_run_params* p, const QcEn
     out->grid = (unsigned)grid;
     out->block = T;
     out->smem = smem;
+    out->scaled = entry->scaled;
+    out->frames_per_cta = F;
     if (grid == 0) return 0;
     if (qc_shape_in_scratch(G)) {
         int rc;
-        const size_t rsz = p->storage == LDPC_STORE_FP32 ? 4 : 2;
-        if ((rc = ensure_cap(&h->d_rmsg, &h->rmsg_cap, grid * F * (size_t)qp.slot_elems * rsz))) return rc;
+        const size_t slot = F * (size_t)qp.slot_elems * (p->storage == LDPC_STORE_FP32 ? 4 : 2);
+        // frames left out: no more CTAs than the scratch of the launch before holds, which is still in use
+        if (out->left_out && h->rmsg_cap >= slot) out->grid = (unsigned)std::min<uint64_t>(grid, h->rmsg_cap / slot);
+        if ((rc = ensure_cap(&h->d_rmsg, &h->rmsg_cap, out->grid * slot))) return rc;
         qp.r_base = h->d_rmsg;
     }
     return 0;
 }
 
+// Decoding passes of run_frames.
+//   SCALED     the scaled kernels where they may be used (qc_scaled_ok): a caller's frames out of their range (llr_scales)
+//              are left out
+//   LEFT_OUT   those frames, on the unscaled kernels
+//   UNSCALED   every frame on the unscaled kernels
+enum Pass : int { UNSCALED, SCALED, LEFT_OUT };
+
 static int launch_qc(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint32_t n, uint64_t first,
-                     const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be, bool scaled) {
+                     const float* d_llr, float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be, Pass pass) {
     QcLaunch L;
-    int rc = prepare_qc(h, p, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, 1.0, &L, scaled);
+    L.left_out = pass == LEFT_OUT;
+    int rc = prepare_qc(h, p, ext, n, first, d_llr, d_post, d_it, d_sf, d_be, 1.0, &L, pass == SCALED);
     if (rc || L.grid == 0) return rc;
+    if (pass == LEFT_OUT) {
+        if (L.frames_per_cta != 1) return LDPC_ENOTSUP;
+        L.qp.redo = 1;
+        L.qp.work += 8;  // a claim counter of its own
+        CU(cudaMemsetAsync(L.qp.work, 0, sizeof(unsigned int), h->stream));
+    }
+    L.qp.left_flag = h->left_flag;
     void* args[] = {&L.qp};
     CU(cudaLaunchKernel(L.fn, dim3(L.grid), dim3(L.block), args, L.smem, h->stream));
     h->launches++;
@@ -826,10 +852,19 @@ static int fill_tally(ldpc_handle* h, const unsigned long long* t, ldpc_tally* o
         out->iter_sum = t[T_ITER_SUM];
         out->unconverged = t[T_UNCONVERGED];
         out->max_iters = t[T_MAX_ITER];
-        out->kernel_ms = ms;
+        out->kernel_ms = h->ms_before + ms;
         out->reserved1 = 0.0f;
         out->bit_errors_sq = t[T_BIT_ERR_SQ];
     }
+    return 0;
+}
+
+// Before another pass over frames of a call: the time the passes so far have taken.
+static int decode_again(ldpc_handle* h) {
+    float ms = 0.0f;
+    CU(cudaStreamSynchronize(h->stream));
+    CU(cudaEventElapsedTime(&ms, h->ev0, h->ev1));
+    h->ms_before += ms;
     return 0;
 }
 
@@ -998,15 +1033,27 @@ static uint64_t copy_chunk(uint64_t off, uint64_t n, uint64_t chunk) {
 // hin (optional): the channel LLRs of the n frames in host memory, copied into d_llr one chunk at a
 // time on the handle's copy stream (bf16 through d_llr16 and the widening kernel) while the
 // previous chunk decodes; chunk <= kMaxLaunchFrames.
+// pass: SCALED or UNSCALED (see Pass); the frames SCALED leaves out are for the caller (run_left_out), but for the first
+// *decoded (if given), which a chunked call has seen to: once a launch has left one out, the frames left out so far
+// and then those of each chunk are decoded behind it, while the next chunk is copied.
 static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64_t n, const float* d_llr,
                       float* d_post, int32_t* d_it, int32_t* d_sf, int32_t* d_be, const HostLlr* hin = nullptr,
-                      uint64_t chunk = kMaxLaunchFrames, bool scaled = true) {
+                      uint64_t chunk = kMaxLaunchFrames, Pass pass = SCALED, uint64_t* decoded = nullptr) {
     int rc;
     if ((rc = reset_counters(h))) return rc;
+    volatile uint32_t* flag = h->left_flag;
+    *flag = 0;
+    bool watch = decoded && hin && chunk < n, behind = false;
+    auto left_out = [&](uint64_t a, uint64_t b) {
+        return launch_qc(h, p, ext, (uint32_t)(b - a), p->first_frame + a, d_llr + a * (uint64_t)(h->N - h->P),
+                         d_post ? d_post + a * (uint64_t)h->N : nullptr, d_it ? d_it + a : nullptr, d_sf ? d_sf + a : nullptr,
+                         d_be ? d_be + a : nullptr, LEFT_OUT);
+    };
     if (n == 0) CU(cudaEventRecord(h->ev0, h->stream));
     const uint64_t ntx = (uint64_t)(h->N - h->P);
     uint32_t cnt = 0;
-    for (uint64_t off = 0; off < n; off += cnt) {
+    int nth = 0;
+    for (uint64_t off = 0; off < n; off += cnt, ++nth) {
         cnt = (uint32_t)(hin && !hin->pageable && chunk < n ? copy_chunk(off, n, chunk) : std::min<uint64_t>(chunk, n - off));
         if (hin) {
             const size_t bytes = (size_t)cnt * ntx * hin->elem;
@@ -1018,8 +1065,11 @@ static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64
             } else {
                 CU(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->cstream));
             }
-            CU(cudaEventRecord(h->cev, h->cstream));
-            CU(cudaStreamWaitEvent(h->stream, h->cev, 0));
+            CU(cudaEventRecord(h->cev[nth % 3], h->cstream));
+            // page-locked copies queue up at once: no more than three ahead, or every chunk would be launched before the
+            // first frame left out is known
+            if (watch && !hin->pageable && nth > 1) CU(cudaEventSynchronize(h->cev[(nth - 2) % 3]));
+            CU(cudaStreamWaitEvent(h->stream, h->cev[nth % 3], 0));
             if (hin->elem == 2) {  // not on the copy stream, where it would wait for SMs and hold up the next copy
                 widen_bf16_kernel<<<h->n_sm * 4, 256, 0, h->stream>>>(h->d_llr16 + off * ntx,
                                                                       const_cast<float*>(d_llr) + off * ntx,
@@ -1035,7 +1085,19 @@ static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64
         int32_t* sf = d_sf ? d_sf + off : nullptr;
         int32_t* be = d_be ? d_be + off : nullptr;
         rc = LDPC_ENOTSUP;
-        if (h->kind == LDPC_KERNEL_QC) rc = launch_qc(h, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be, scaled);
+        if (h->kind == LDPC_KERNEL_QC) {
+            if (watch && !behind && *flag) {
+                rc = left_out(0, off);
+                if (rc && rc != LDPC_ENOTSUP) return rc;
+                behind = rc == 0;
+                watch = behind;
+            }
+            rc = launch_qc(h, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be, pass);
+            if (!rc && behind) {
+                if ((rc = left_out(off, off + cnt))) return rc;
+                *decoded = off + cnt;
+            }
+        }
         if (rc == LDPC_ENOTSUP && p->algo == LDPC_ALGO_WAMIN)
             return fail(LDPC_ENOTSUP, "the weighted decoder is not built for Z=%d D=%d with storage %d", h->Z, h->D,
                         p->storage);
@@ -1054,7 +1116,7 @@ static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64
             if (sh[3] != GEN_LAYOUT_WARP)
                 rc = launch_general_step(&h->gen, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be,
                                          h->d_tally, h->d_hist, h->hist_bins, h->d_work, h->n_sm, h->stream, g_err,
-                                         h->d_snr, scaled && !ext && qc_scaled_ok(p, ext));
+                                         h->d_snr, pass == SCALED && !ext && qc_scaled_ok(p, ext));
             if (rc == LDPC_ENOTSUP)
                 rc = launch_general(&h->gen, p, ext, cnt, p->first_frame + off, llr, post, it, sf, be, h->d_tally,
                                     h->d_hist, h->hist_bins, h->d_work, h->n_sm, h->stream, g_err, h->d_snr);
@@ -1067,16 +1129,33 @@ static int run_frames(ldpc_handle* h, const ldpc_run_params* p, bool ext, uint64
     return 0;
 }
 
+// The frames that a SCALED pass over caller-supplied LLRs has left out, of frames first to n - 1; the counters go on.
+// LDPC_ENOTSUP: not built (the caller runs an UNSCALED pass).
+static int run_left_out(ldpc_handle* h, const ldpc_run_params* p, uint64_t first, uint64_t n, const float* d_llr, float* d_post,
+                        int32_t* d_it, int32_t* d_sf, int32_t* d_be) {
+    int rc;
+    if ((rc = decode_again(h))) return rc;
+    CU(cudaEventRecord(h->ev0, h->stream));
+    for (uint64_t off = first; off < n && !rc; off += kMaxLaunchFrames)
+        rc = launch_qc(h, p, true, (uint32_t)std::min<uint64_t>(kMaxLaunchFrames, n - off), p->first_frame + off,
+                       d_llr + off * (uint64_t)(h->N - h->P), d_post ? d_post + off * (uint64_t)h->N : nullptr, d_it + off,
+                       d_sf + off, d_be + off, LEFT_OUT);
+    CU(cudaEventRecord(h->ev1, h->stream));
+    return rc;
+}
+
 extern "C" int ldpc_run_chunk(ldpc_handle* h, const ldpc_run_params* p, ldpc_tally* out) {
     int rc;
     if ((rc = check_params(h, p))) return rc;
     CU(cudaSetDevice(h->device));
+    h->ms_before = 0.0f;
     if ((rc = run_frames(h, p, false, p->n_frames, nullptr, nullptr, nullptr, nullptr, nullptr))) return rc;
     if ((rc = read_tally(h, out))) return rc;
     if (!h->h_tally[T_OUT_OF_RANGE]) return 0;
     // a frame's values left the scaled kernels' range: the same frames on the unscaled ones
+    if ((rc = decode_again(h))) return rc;
     if ((rc = run_frames(h, p, false, p->n_frames, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, kMaxLaunchFrames,
-                         false)))
+                         UNSCALED)))
         return rc;
     return read_tally(h, out);
 }
@@ -1116,15 +1195,24 @@ static int decode_small(ldpc_handle* h, const ldpc_run_params* p, const void* ll
     int32_t *d_sf = d_it + n, *d_be = d_sf + n;
     float* d_post = reinterpret_cast<float*>(d_be + n);
     const size_t post_bytes = post ? n * h->N * sizeof(float) : 0;
-    // (scaled; again on the unscaled kernels if the LLRs are out of the scaled ones' range)
-    for (int scaled = 1; scaled >= 0; --scaled) {
-        if ((rc = run_frames(h, p, true, n, d_llr, post ? d_post : nullptr, d_it, d_sf, d_be, nullptr, kMaxLaunchFrames,
-                             scaled != 0)))
-            return rc;
+    // scaled; then, where LLRs or values are out of the scaled kernels' range, the frames left out or all again
+    h->ms_before = 0.0f;
+    const unsigned long long* t = reinterpret_cast<const unsigned long long*>(h->h_small);
+    for (Pass pass = SCALED;;) {
+        rc = pass == LEFT_OUT ? run_left_out(h, p, 0, n, d_llr, post ? d_post : nullptr, d_it, d_sf, d_be)
+                              : run_frames(h, p, true, n, d_llr, post ? d_post : nullptr, d_it, d_sf, d_be, nullptr,
+                                           kMaxLaunchFrames, pass);
+        if (pass == LEFT_OUT && rc == LDPC_ENOTSUP) {
+            pass = UNSCALED;
+            continue;
+        }
+        if (rc) return rc;
         CU(cudaMemcpyAsync(h->h_small, h->d_tally, TALLY_WORDS * 8 + 3 * n * sizeof(int32_t) + post_bytes,
                            cudaMemcpyDeviceToHost, h->stream));
         CU(cudaStreamSynchronize(h->stream));
-        if (!reinterpret_cast<const unsigned long long*>(h->h_small)[T_OUT_OF_RANGE]) break;
+        if (pass == UNSCALED || (!t[T_OUT_OF_RANGE] && t[T_FRAMES] == n)) break;
+        pass = t[T_OUT_OF_RANGE] ? UNSCALED : LEFT_OUT;
+        if (pass == UNSCALED && (rc = decode_again(h))) return rc;
     }
     const unsigned char* o = h->h_small + TALLY_WORDS * 8;
     if (iters) memcpy(iters, o, n * sizeof(int32_t));
@@ -1234,8 +1322,9 @@ static int decode_host(ldpc_handle* h, const ldpc_run_params* p, const void* llr
     }
     if (!h->cstream && cudaStreamCreateWithFlags(&h->cstream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(LDPC_EIO, "copy stream creation failed");
-    if (!h->cev && cudaEventCreateWithFlags(&h->cev, cudaEventDisableTiming) != cudaSuccess)
-        return fail(LDPC_EIO, "copy event creation failed");
+    for (cudaEvent_t& e : h->cev)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
+            return fail(LDPC_EIO, "copy event creation failed");
     // Large calls copy the LLRs in chunks on the copy stream, so that the decoding of one chunk
     // overlaps the copy of the next; small ones are one chunk.
     constexpr uint64_t kMinChunk = 8192;
@@ -1245,15 +1334,27 @@ static int decode_host(ldpc_handle* h, const ldpc_run_params* p, const void* llr
     int32_t* d_it = h->d_frame_out;
     int32_t* d_sf = d_it ? d_it + nb : nullptr;
     int32_t* d_be = d_sf ? d_sf + nb : nullptr;
+    uint64_t decoded = 0;
+    h->ms_before = 0.0f;
     if ((rc = run_frames(h, &q, true, nb, h->d_llr, post ? h->d_post : nullptr, d_it, d_sf, d_be,
-                         nb ? &hin : nullptr, chunk)))
+                         nb ? &hin : nullptr, chunk, SCALED, &decoded)))
         return rc;
+    auto rest = [&] { return run_left_out(h, &q, decoded, nb, h->d_llr, post ? h->d_post : nullptr, d_it, d_sf, d_be); };
+    // before a copy of many posteriors (0.3 ms and more; the wait 10 us) the frames left out; else only after the
+    // outputs have been copied, which then are copied again
+    constexpr size_t kLook = 16u << 20;
+    if (post && nb * h->N * sizeof(float) >= kLook) {
+        CU(cudaStreamSynchronize(h->stream));
+        if (*static_cast<volatile uint32_t*>(h->left_flag) && (rc = rest()) && rc != LDPC_ENOTSUP) return rc;
+    }
     if ((rc = host_outputs(h, nb, plain, post, iters, synd_fail, bit_errors, out))) return rc;
-    if (!nb || !h->h_tally[T_OUT_OF_RANGE]) return 0;
-    // the LLRs, now on the device, are out of the scaled kernels' range
-    if ((rc = run_frames(h, &q, true, nb, h->d_llr, post ? h->d_post : nullptr, d_it, d_sf, d_be, nullptr, kMaxLaunchFrames,
-                         false)))
-        return rc;
+    if (!nb || (!h->h_tally[T_OUT_OF_RANGE] && h->h_tally[T_FRAMES] == nb)) return 0;
+    rc = h->h_tally[T_OUT_OF_RANGE] ? LDPC_ENOTSUP : rest();
+    if (rc == LDPC_ENOTSUP) {  // values have left the scaled kernels' range: all again, the LLRs now on the device
+        if ((rc = decode_again(h))) return rc;
+        rc = run_frames(h, &q, true, nb, h->d_llr, post ? h->d_post : nullptr, d_it, d_sf, d_be, nullptr, kMaxLaunchFrames, UNSCALED);
+    }
+    if (rc) return rc;
     return host_outputs(h, nb, plain, post, iters, synd_fail, bit_errors, out);
 }
 
@@ -1447,9 +1548,13 @@ static int batch_run(ldpc_batch* b, const ldpc_run_params* params, const float* 
 extern "C" int ldpc_batch_run(ldpc_batch* b, const ldpc_run_params* params, const float* share, ldpc_tally* out,
                               float* graph_ms) {
     bool far = false;
-    const int rc = batch_run(b, params, share, out, graph_ms, true, &far);
+    float ms = 0.0f, again = 0.0f;
+    int rc = batch_run(b, params, share, out, &ms, true, &far);
     // a frame's values left the scaled kernels' range: the same frames on the unscaled ones
-    return rc || !far ? rc : batch_run(b, params, share, out, graph_ms, false, &far);
+    if (!rc && far) rc = batch_run(b, params, share, out, &again, false, &far);
+    if (!rc && graph_ms) *graph_ms = ms + again;
+    for (size_t i = 0; !rc && out && far && i < b->hs.size(); ++i) out[i].kernel_ms += ms;
+    return rc;
 }
 
 static int batch_run(ldpc_batch* b, const ldpc_run_params* params, const float* share, ldpc_tally* out, float* graph_ms,

@@ -78,6 +78,8 @@ struct QcParams {
     float circ_c[4];
     float circ_damping;
     int32_t circ_sfpu;
+    int32_t redo;         // caller-supplied LLRs, unscaled kernels: only the frames the scaled kernel before has left out
+    uint32_t* left_flag;  // set to 1 by a scaled kernel that leaves out a frame (host memory; optional)
 };
 
 // Host side (ldpc_capi.cu).  The quasi-cyclic structure of a row table, found without allocating; the default
@@ -104,7 +106,8 @@ __host__ __device__ constexpr int qc_edge_slot(int l, int e, int D) {
 enum TallyWord : int {
     T_FRAMES = 0, T_BIT_ERR, T_FRAME_ERR, T_ITER_SUM, T_UNCONVERGED, T_MAX_ITER, T_BIT_ERR_SQ,
     T_OUT_OF_RANGE,  // set by a scaled kernel whose values left its range (LLR_SCALE)
-    TALLY_WORDS = 8
+    T_LEFT_OUT,      // frames whose caller-supplied LLRs a scaled kernel does not decode (llr_scales)
+    TALLY_WORDS
 };
 
 template <int MODE> struct LTraits;
@@ -637,7 +640,7 @@ __device__ __forceinline__ void ot_load(const uint32_t* tab, int t, int* idx) {
     if constexpr (rem & 1) idx[d - 1] = (int)tab[T * (c4 + (rem >= 2 ? 2 : 0)) + t];
 }
 
-// Whether a caller's channel LLR v may be decoded as x = v LLR_SCALE: below 2^20 (and not NaN), and x exact as it is
+// Whether a caller's channel LLR v may be decoded (scaled kernels leave out the frames of others) as x = v LLR_SCALE: below 2^20 (and not NaN), and x exact as it is
 // stored.  A bf16 subnormal has fewer bits than the bf16 of v, so with bf16 storage x is zero or normal (|v| >=
 // 2^-76); every value computed from such LLRs is then a multiple of 2^-83, as bf16 at LLR_SCALE a multiple of its
 // smallest subnormal.  In fp32 the product is exact down to the last bit of its subnormals.
@@ -671,7 +674,8 @@ __device__ __forceinline__ int qc_shift(const QcParams& p, int l, int e) {
 // only for a matrix whose descriptors are those).
 // SC: the frames are decoded at LLR_SCALE (Approximate-Min*, or the simulation of the circulant engine's decoder;
 // fp32 or bf16 storage, no clips): the same values but for the scale, one instruction less per min* step.  A
-// caller's LLR out of range (llr_scales) is reported in the tally.
+// frame with a caller's LLR out of range (llr_scales) is left out, and counted in the tally; a launch of the unscaled
+// kernel with p.redo decodes those.
 // ROLL (layout 7, global messages only): the eight degree-D layers run as one loop that is not
 // unrolled, each row's descriptors read from the kernel parameters by layer index.  The unrolled
 // body of a degree-18 code is tens of KB of instructions; with one-warp CTAs whose warps are
@@ -691,12 +695,15 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
     constexpr bool CIRC = ALGO == ALGO_CIRC;
     static_assert(!SC || (!CLIP && !PAIR && MODE != STORE_FP16 && (ALGO == ALGO_AMIN || (CIRC && !EXT))),
                   "scaled decoding: no clips, no fp16 messages");
+    static_assert(!SC || !EXT || F == 1, "frames are left out one at a time");
+    constexpr bool REDO = EXT && !SC && F == 1 && ALGO == ALGO_AMIN && MODE != STORE_FP16;  // p.redo is looked at
     static_assert(!ROLL || (RG && FIX < 0 && !CIRC), "the rolled layer loop: global messages, parameter descriptors");
     static_assert(!CIRC || (D == 6 && !CLIP && !PAIR), "the circulant engine's decoder: degrees 3 and 6, no clips");
     using SV = SlotView<MODE, PAIR>;
     using LT = LTraits<MODE>;
     using LE = typename LT::T;
 
+    if (REDO && p.redo && p.tally[T_LEFT_OUT] == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int N = p.n_vars;
     const int nblk = N / Z;
@@ -763,6 +770,15 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                     }
             }
             __syncthreads();
+            if (REDO && p.redo && s_fid[0] != 0xFFFFFFFFu) {  // a frame that was not left out: the next one
+                bool left = false;
+                for (int i = tid; i < p.n_tx; i += T) {
+                    const float v = p.llr_in[(size_t)s_fid[0] * p.n_tx + i];
+                    left |= !llr_scales<MODE>(v, v * LLR_SCALE);
+                }
+                if (!__syncthreads_or((int)left)) continue;
+            }
+            bool far = false;  // SC: an LLR of the frame is out of range
 #pragma unroll
             for (int f = 0; f < F; ++f) {
                 if (!(need & (1u << f))) continue;
@@ -781,7 +797,6 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                 const int nq = p.n_tx >> 2;
                 if (EXT) {
                     const float4* src = reinterpret_cast<const float4*>(p.llr_in + (size_t)fid[f] * p.n_tx);
-                    bool far = false;
                     for (int qd = tid; qd < nq; qd += T) {
                         const float4 v4 = src[qd];
                         float v[4] = {v4.x, v4.y, v4.z, v4.w};
@@ -796,7 +811,6 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                             L.st(4 * qd + k, x);
                         }
                     }
-                    if (SC && far) p.tally[T_OUT_OF_RANGE] = 1ull;
                 } else {
                     const uint64_t gf = p.first_frame + fid[f];
                     float ch_mu = p.mu, ch_sigma = p.sigma;
@@ -828,7 +842,19 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
                 for (int i = p.n_tx + tid; i < N; i += T) L.st(i, 0.0f);
             }
             need = 0;
-            __syncthreads();
+            if constexpr (SC && EXT) {
+                if (__syncthreads_or((int)far)) {  // the frame is left out
+                    if (tid == 0) {
+                        s_tally[T_LEFT_OUT] += 1;
+                        if (p.left_flag) *reinterpret_cast<volatile uint32_t*>(p.left_flag) = 1;
+                    }
+                    need = 1;
+                    act = 0;
+                    continue;
+                }
+            } else {
+                __syncthreads();
+            }
         }
         if (!act) break;
 
@@ -1133,6 +1159,7 @@ __global__ void __launch_bounds__(Z / R, B) qc_decode_kernel(const __grid_consta
     if constexpr (SC) {
         if (hi >= 1.0f) p.tally[T_OUT_OF_RANGE] = 1ull;
         if (tid != 0) return;
+        if (EXT && s_tally[T_LEFT_OUT]) atomicAdd(&p.tally[T_LEFT_OUT], s_tally[T_LEFT_OUT]);
         t_frames = s_tally[T_FRAMES];
         t_be = s_tally[T_BIT_ERR];
         t_be2 = s_tally[T_BIT_ERR_SQ];

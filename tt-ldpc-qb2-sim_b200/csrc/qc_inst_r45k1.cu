@@ -60,8 +60,9 @@ static const QcEntry qc_r45k1[] = {
     // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 16),
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 24),
-    // fp32 caller-supplied LLRs at LLR_SCALE (the unscaled counterpart is the larger cap)
-    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 20),
+    // fp32 caller-supplied LLRs at LLR_SCALE (the unscaled counterpart is the larger cap): us for 8000 / 300 frames with 16
+    // CTAs' registers 293 / 65.5, 18 310 / 67.6, 20 310 / 65.5, 22 329 / 69
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 16),
 };
 LDPC_QC_REGISTER(qc_r45k1)
 
@@ -73,7 +74,7 @@ LDPC_QC_REGISTER(qc_r45k1)
 static const QcDefault qc_r45k1_default[] = {
     {32, 18, STORE_BF16, -1, 0, 1, 1, 16, 7},
     {32, 18, STORE_FP16, -1, 0, 1, 1, 16, 7},
-    {32, 18, STORE_FP32, -1, 0, 1, 1, 20, 7},  // (caller-supplied LLRs only)
+    {32, 18, STORE_FP32, -1, 0, 1, 1, 16, 7},  // (caller-supplied LLRs only)
     {32, 18, STORE_FP32, -1, 0, 1, 1, 24, 7},
 };
 LDPC_QC_DEFAULTS(qc_r45k1_default)
