@@ -1224,7 +1224,10 @@ static int decode_small(ldpc_handle* h, const ldpc_run_params* p, const void* ll
 
 // Device -> host copy into a pageable array through the pinned ring: while the host copies one piece out of its
 // slot (threads share the work, and the page faults of a fresh array), the next piece travels.  Only where the ring is
-// there already, for pageable LLRs: pinning its 96 MB takes some 50 ms, the copy of 41 MB by the driver 0.4 ms more.
+// there already, for pageable LLRs (pinning its 96 MB takes some 50 ms), and from kRingPost on; whole calls, ms, through
+// the ring and by the driver's copy, r1/2 K=1024 fp32: 12 MB 2.53, 2.35; 16 MB 3.46, 3.22; 20 MB 3.78, 4.01; 28 MB 4.09,
+// 4.87; 39 MB 7.5, 12.0.  K=4096 and K=16384 cross between the same sizes.
+constexpr size_t kRingPost = 18u << 20;
 static int unstage_d2h(ldpc_handle* h, char* dst, const char* src, size_t bytes) {
     int rc;
     if ((rc = stage_alloc(h))) return rc;
@@ -1261,12 +1264,12 @@ static int host_outputs(ldpc_handle* h, size_t nb, bool plain, float* post, int3
     if (!nb) return read_tally(h, out);
     int32_t *d_it = h->d_frame_out, *d_sf = d_it + nb, *d_be = d_sf + nb;
     bool ring = false;
-    if (post && host_memory(post, &ring) && ring && h->stage[ldpc_handle::kStageSlots - 1]) {
-        if ((rc = unstage_d2h(h, reinterpret_cast<char*>(post), reinterpret_cast<const char*>(h->d_post),
-                              nb * h->N * sizeof(float))))
+    const size_t post_bytes = nb * h->N * sizeof(float);
+    if (post && post_bytes >= kRingPost && host_memory(post, &ring) && ring && h->stage[ldpc_handle::kStageSlots - 1]) {
+        if ((rc = unstage_d2h(h, reinterpret_cast<char*>(post), reinterpret_cast<const char*>(h->d_post), post_bytes)))
             return rc;
     } else if (post) {
-        CU(cudaMemcpyAsync(post, h->d_post, nb * h->N * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        CU(cudaMemcpyAsync(post, h->d_post, post_bytes, cudaMemcpyDeviceToHost, h->stream));
     }
     // the per-frame counts: through the pinned buffer where it takes a few copies, else one copy per array
     constexpr size_t kPiece = (ldpc_handle::kSmallHost - TALLY_WORDS * 8) / sizeof(int32_t);
