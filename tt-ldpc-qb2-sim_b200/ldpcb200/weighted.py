@@ -196,7 +196,7 @@ class SoftplusRows(torch.autograd.Function):
     def backward(ctx, g):
         (x,) = ctx.saved_tensors
         # a gradient that is itself differentiated, or one of a batch of gradients (it has no storage)
-        if torch.is_grad_enabled() or not _one_pass(x) or not torch._C._has_storage(g):
+        if torch.is_grad_enabled() or not _one_pass(x) or not _has_storage(g):
             return -g.unsqueeze(-1) * torch.sigmoid(-x)
         g = g.contiguous()
         gx = torch.empty_like(x)
@@ -211,12 +211,27 @@ def _one_pass(x: torch.Tensor) -> bool:
     """Whether softplus(-x).sum(-1) runs on the one-pass kernels: plain contiguous float32 CUDA rows, and
     nothing that looks into the operations (function transforms, forward-mode differentiation, tracing,
     compilation, dispatch modes) is active; everything else takes the library's operations."""
-    return (type(x) in (torch.Tensor, torch.nn.Parameter) and not torch._C._are_functorch_transforms_active()
-            and torch.autograd.forward_ad._current_level < 0 and not torch.jit.is_tracing()
-            and not torch.compiler.is_compiling() and torch._C._len_torch_dispatch_stack() == 0
-            and torch._C._len_torch_function_stack() == 0 and x.is_cuda and x.dtype == torch.float32 and x.dim() > 0
-            and x.numel() > 0 and x.shape[-1] % 4 == 0 and x.shape[-1] < 2 ** 31 and x.is_contiguous()
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and _unobserved() and x.is_cuda and x.dtype == torch.float32
+            and x.dim() > 0 and x.numel() > 0 and x.shape[-1] % 4 == 0 and x.shape[-1] < 2 ** 31 and x.is_contiguous()
             and not x.is_neg() and x.data_ptr() % 16 == 0)
+
+
+def _unobserved() -> bool:
+    """Whether no function transform, forward-mode level, trace, compilation or mode is active.  torch has no public
+    queries for most of these; where a release lacks one of them the answer is no."""
+    try:
+        return (not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+                and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+                and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
+    except AttributeError:
+        return False
+
+
+def _has_storage(g: torch.Tensor) -> bool:
+    try:
+        return torch._C._has_storage(g)
+    except AttributeError:
+        return False
 
 
 def softplus_rows(post: torch.Tensor) -> torch.Tensor:
