@@ -27,10 +27,10 @@ static const QcEntry qc_circ[] = {
 };
 LDPC_QC_REGISTER(qc_circ)
 
-// Defaults (us of the kernel at 440 / 100000 frames, 25000 for K = 4096, 2.04 dB): bf16 layout 6 54.4 / 6734,
-// offset table 55.6 / 6934, parameters 56.4 / 8023; fp32 44.6 / 5315 against 46.4 / 5917; K = 4096 148 / 6911
-// against 164 / 8017, but one frame 56.7 against 52.5.  K = 16384 keeps the parameter kernel: with the
-// descriptors compiled in it spills and takes 1.14 times as long.
+// Defaults.  us of the kernel at 440 / 5000 / 100000 frames (440 / 1500 / 25000 for K = 4096), 2.04 dB, all shapes in one run: bf16
+// layout 6 51.9 / 334 / 6160, offset table 57.3 / 350 / 6374, parameters 57.4 / 420 / 7964; fp32 37.8 / 254 / 4654 and 45.1 / 316 /
+// 5888; K = 4096 135 / 428 / 6440 and 167 / 524 / 8011.  K = 16384 keeps the parameter kernel: with the descriptors compiled in
+// it spills and took 1.14 times as long.
 static const QcDefault qc_circ_default[] = {
     {128, 6, STORE_BF16, ALGO_CIRC, 0, 1, 1, 5, 6},
     {128, 6, STORE_BF16, ALGO_CIRC, 440, 1, 1, 0, 2},

@@ -68,17 +68,17 @@ static const QcEntry qc_k16[] = {
 };
 LDPC_QC_REGISTER(qc_k16)
 
-// Default shapes (us of the kernel at 1 / 100 / 440 / 6250 frames, threshold + 1.4 dB): the descriptors compiled in
-//   r1/2 bf16 187.8 / 189.4 / 473.3 / 6102, parameters 204.0 / 206.1 / 528.8 / 6812; fp16 184.5 / 190.8 / 535.5 / 6988 against
-//        199.0 / 205.0 / 575.8 / 7539
-//   r2/3 bf16 110.7 / 128.3 / 309.5 / 3948 (cap 2 3978), parameters 110.9 / 128.1 / 353.6 / 4603; fp16 cap 2 111.3 / 129.2 / 358.5 /
-//        4672 against 115.0 / 133.3 / 369.0 / 4800
-//   r4/5 bf16 cap 2 90.4 / 108.7 / 241.7 / 3026, uncapped 86.2 / 102.6 / 260.4 / 3372, parameters 88.2 / 106.5 / 272.5 / 3507;
-//        fp16 cap 2 92.4 / 110.9 / 243.9 / 3050 against 88.2 / 106.6 / 274.5 / 3522
+// Default shapes.  us of the kernel at 1 / 100 / 440 / 6250 frames, threshold + 1.4 dB, all shapes in one run: the descriptors
+// compiled in
+//   r1/2 bf16 147 / 187 / 451 / 5816, parameters 165 / 210 / 527 / 6804; fp16 170 / 191 / 532 / 6984 and 182 / 206 / 573 / 7539
+//   r2/3 bf16 cap 2 111 / 127 / 297 / 3767, uncapped 108 / 123 / 331 / 4278, parameters 114 / 132 / 356 / 4605; fp16 cap 2 113 / 133 / 360 /
+//        4669, parameters 115 / 136 / 370 / 4793
+//   r4/5 bf16 cap 2 86.0 / 101 / 231 / 2919, uncapped 88.1 / 102 / 231 / 2917, parameters 88.1 / 104 / 270 / 3520; fp16 cap 2 92.2 / 109 / 244 /
+//        3055, parameters 88.9 / 105 / 271 / 3537
 // Scaled kernels add up their rows' magnitudes (`hi` of row_update), which takes r2/3 bf16 without a cap past 64 registers, to
 // one CTA an SM: 3750 frames 2270 us before, 2598 since, cap 2 2285; caller-supplied LLRs, 500 frames, 367, 423, 378.
-// Min-sum and the clips have only these shapes: bf16 r1/2 192.7 / 192.9 / 455.0 and 207.0 / 209.0 / 526.6, r2/3 112.9 / 114.8 /
-// 282.9 and 121.0 / 139.5 / 344.4, r4/5 80.0 / 94.5 / 213.1 and 94.3 / 113.0 / 260.2 (the general kernel before).
+// Min-sum and the clips have only these shapes: bf16 r1/2 156 / 195 / 455 / 5853 and 166 / 211 / 526 / 6750, r2/3 97.2 / 128 / 293 /
+// 3646 and 124 / 142 / 343 / 4335, r4/5 77.8 / 96.3 / 212 / 2604 and 94.2 / 111 / 282 / 3261 (the general kernel before).
 static const QcDefault qc_k16_default[] = {
     {2048, 6, STORE_BF16, -1, 0, 4, 1, 0, 5},
     {2048, 6, STORE_FP16, -1, 0, 4, 1, 0, 5},

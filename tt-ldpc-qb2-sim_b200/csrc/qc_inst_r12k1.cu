@@ -108,21 +108,19 @@ static const QcEntry qc_r12k1[] = {
 };
 LDPC_QC_REGISTER(qc_r12k1)
 
-// Default shapes (us of the kernel at 1 / 440 / 1500 / 100000 frames, 2.04 dB, Approximate-Min*).  Few frames
-// wait for the slowest of them, where fewer registers per thread do not help; with many, resident warps and
-// instructions decide.  Layout 6 cap 5 is ahead at both ends since its min* step is one instruction shorter
-// (amin_step_scaled): bf16 at 1 / 440 / 1500 / 5000 / 100000 frames 21.5 / 43.2 / 98 / 276 / 4982 against cap 8 25.6 / 54.1 /
-// 109.5 / 284 / 5067, caller-supplied LLRs (8000 frames) 429 against 445; fp16 (20.5 / 48.2 / 102.4) / 285 / 5102 against
-// layout 2 cap 6 289 / 5173.  The figures below were taken before that, of one run each.
-//   bf16: layout 0 cap 5 25.0 / 47.5 / 110.8 / 5831, layout 6 cap 8 27.6 / 50.2 / 108.6 / 5269, layout 2 cap 8 - / 53.5 / 109.0 / 5335,
-//         (1,1,0,0) 26.9 / 52.2 / 119.0 / 6268
-//   fp16: layout 0 cap 5 23.5 / 46.3 / 110.8 / 5780, layout 2 cap 6 26.8 / 47.5 / 104.9 / 5171, layout 6 cap 6 24.9 / 45.4 / 104.8 /
-//         5218, (1,1,0,0) 24.9 / 49.2 / 114.0 / 5966
-//   fp32: layout 6 21.0 / 39.3 / 95.6 / 5057, its cap 5 22.8 / 39.1 / 92.5 / 4664, layout 2 cap 5 26.8 / 45.4 / 94.7 / 4678,
-//         (1,1,0,0) 22.8 / 43.3 / 96.4 / 5143
-//   normalised min-sum bf16: layout 6 cap 8 27.9 / 51.6 / 107.4 / 5013 against 22.8 / 48.5 / 109.8 / 5757; with clips 30.0 /
-//   55.6 / 125.2 / 6028 against 29.0 / 56.2 / 135.1 / 6915; weighted fp32: layout 2 37.2 / 55.8 / 121.3 / 2396 (40000)
-//   against 35.1 / 53.6 / 120.9 / 2483, its cap 5 2484; fp16: cap 5 35.9 / 57.7 / 129.1 / 2589 against 2799
+// Default shapes.  us of the kernel at 1 / 440 / 1500 / 5000 / 100000 frames, 2.04 dB, all shapes in one run.  Few frames wait for
+// the slowest of them, where fewer registers a thread do not help; with many, resident warps and instructions decide.
+//   bf16: layout 6 cap 5 22.4 / 45.1 / 98.2 / 277 / 5007, cap 8 24.5 / 50.0 / 103 / 284 / 5084, layout 2 25.6 / 53.2 / 106 / 289 / 5141,
+//         layout 0 cap 5 23.6 / 49.2 / 109 / 311 / 5675, (1,1,0,0) 25.6 / 55.3 / 120 / 341 / 6268
+//   fp16: layout 6 cap 5 20.5 / 43.0 / 98.3 / 279 / 5103, cap 6 22.5 / 45.9 / 104 / 289 / 5220, layout 2 cap 6 24.5 / 49.1 / 104 / 289 /
+//         5171, (1,1,0,0) 23.6 / 51.0 / 114 / 324 / 5960
+//   fp32: layout 6 19.1 / 38.9 / 86.0 / 239 / 4356, its cap 5 19.1 / 38.9 / 84.0 / 236 / 4252, layout 2 cap 5 22.5 / 43.0 / 94.1 / 254 /
+//         4530, (1,1,0,0) 21.2 / 43.8 / 99.1 / 281 / 5140
+//   normalised min-sum bf16: layout 6 cap 8 21.2 / 49.3 / 102 / 281 / 5006, (1,1,0,0) 18.5 / 45.1 / 106 / 312 / 5750; with clips 26.5 /
+//         56.2 / 122 / 335 / 6499 and 26.6 / 56.2 / 131 / 374 / 7405
+//   weighted fp32: layout 2 31.7 / 61.4 / 122 / 335 / 6011, (1,1,0,0) 28.7 / 58.0 / 120 / 342 / 6241; fp16: cap 5 30.7 / 61.4 / 127 / 356 /
+//         6499, (1,1,0,0) 31.6 / 63.5 / 135 / 384 / 7037
+// The other lines are for options or matrices the first of their storage is not built for.
 static const QcDefault qc_r12k1_default[] = {
     {128, 6, STORE_FP32, ALGO_WAMIN, 1500, 1, 1, 0, 2},
     {128, 6, STORE_FP32, ALGO_WAMIN, 0, 1, 1, 0, 0},

@@ -44,12 +44,12 @@ static const QcEntry qc_r12k4[] = {
 };
 LDPC_QC_REGISTER(qc_r12k4)
 
-// Default shapes (us of the kernel at 1 / 100 / 440 / 25000 frames, 2.04 dB): up to one frame per SM the
-// uncapped kernel is as fast; above, layout 6 holds two CTAs per SM
-//   bf16: layout 6 47.4 / 57.5 / 121.8 / 5673, (1,1,0,0) 47.3 / 58.7 / 143.7 / 6885; min-sum (12500 frames) 48.5 / 59.7 /
-//         121.0 / 2226 against 48.2 / 57.6 / 139.6 / 2672; with clips 53.4 / 64.7 / 139.6 / 2637 against 55.6 / 67.7 / 168.1 / 3246
-//   fp16: layout 6 47.1 / 53.3 / 120.0 / 5712, (1,1,0,0) 46.2 / 53.4 / 134.3 / 6631
-//   fp32: layout 6 39.2 / 45.3 / 117.0 / 5565, layout 2 43.2 / 49.4 / 122.2 / 5632, (1,1,0,0) 43.2 / 49.4 / 129.2 / 6122
+// Default shapes.  us of the kernel at 1 / 100 / 440 / 1500 / 25000 frames, 2.04 dB, all shapes in one run: up to one frame per SM
+// the uncapped kernel is about as fast; above, layout 6 holds two CTAs per SM
+//   bf16: layout 6 42.0 / 51.9 / 120 / 362 / 5503, (1,1,0,0) 43.0 / 53.3 / 143 / 446 / 6886; min-sum 44.9 / 54.2 / 121 / 366 / 5504 and
+//         43.9 / 54.1 / 138 / 429 / 6633; with clips 47.1 / 59.4 / 141 / 436 / 6521 and 50.0 / 61.4 / 167 / 521 / 8062
+//   fp16: layout 6 41.0 / 53.2 / 123 / 385 / 5714, (1,1,0,0) 41.9 / 53.2 / 137 / 430 / 6628
+//   fp32: layout 6 34.5 / 43.0 / 110 / 340 / 5212, layout 2 39.6 / 47.8 / 117 / 355 / 5401, (1,1,0,0) 39.6 / 49.9 / 127 / 398 / 6123
 static const QcDefault qc_r12k4_default[] = {
     {512, 6, STORE_BF16, -1, 200, 1, 1, 2, 6},
     {512, 6, STORE_FP16, -1, 200, 1, 1, 2, 6},

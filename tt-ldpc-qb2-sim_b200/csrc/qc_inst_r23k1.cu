@@ -54,13 +54,13 @@ static const QcEntry qc_r23k1[] = {
 };
 LDPC_QC_REGISTER(qc_r23k1)
 
-// Default shapes (us of the kernel at 1 / 440 / 5000 / 100000 frames, 2.85 dB):
-//   bf16: layout 6 29.1 / 64.8 / 241.0 / 4415, layout 7 33.0 / 74.1 / 238.9 / 3920, layout 2 30.9 / 68.0 / 270.7 / 4930,
-//         (1,1,0,0) 31.0 / 75.1 / 300.2 / 5640; min-sum layout 6 22.9 / 75.0 / 187.7 / 3238, layout 7 25.9 / 100.4 / 250.2 /
-//         3782, (1,1,0,0) 28.9 / 105.4 / 244.6 / 4332; with clips layout 6 28.7 / 69.7 / 288.1 / 5301, layout 7 35.0 / 77.2 /
-//         261.5 / 4380, (1,1,0,0) 32.1 / 81.2 / 354.5 / 6727
-//   fp16: layout 2 35.2 / 75.1 / 264.4 / 4823, (1,1,0,0) 33.1 / 77.1 / 295.2 / 5584
-//   fp32: layout 2 29.2 / 59.8 / 215.4 / 3867, layout 7 31.9 / 73.9 / 227.6 / 3580, (1,1,0,0) 26.9 / 68.0 / 281.9 / 5184
+// Default shapes.  us of the kernel at 1 / 440 / 1500 / 5000 / 100000 frames, 2.85 dB, all shapes in one run:
+//   bf16: layout 6 25.5 / 45.1 / 82.8 / 232 / 4240, layout 7 27.7 / 49.2 / 89.0 / 224 / 3659, layout 2 28.7 / 50.2 / 90.1 / 251 / 4508,
+//         (1,1,0,0) 30.7 / 55.3 / 104 / 309 / 5676; min-sum layout 6 19.5 / 39.8 / 70.7 / 187 / 3258, layout 7 23.5 / 51.2 / 90.1 / 238 /
+//         3826, (1,1,0,0) 24.5 / 52.1 / 96.2 / 255 / 4472; with clips layout 6 28.7 / 52.1 / 1053 / 1178 / 6284, layout 7 30.7 / 57.3 /
+//         1162 / 1312 / 5465, (1,1,0,0) 30.8 / 59.4 / 1164 / 1399 / 7984
+//   fp16: layout 2 29.4 / 51.2 / 96.3 / 263 / 4828, (1,1,0,0) 30.7 / 53.4 / 104 / 299 / 5569
+//   fp32: layout 2 25.4 / 42.0 / 77.8 / 225 / 3594, layout 7 28.6 / 50.1 / 87.0 / 247 / 3438, (1,1,0,0) 26.6 / 47.9 / 101 / 297 / 5181
 static const QcDefault qc_r23k1_default[] = {
     {64, 10, STORE_BF16, ALGO_NMS, 0, 1, 1, 0, 6},
     {64, 10, STORE_BF16, -1, 5000, 1, 1, 16, 7},

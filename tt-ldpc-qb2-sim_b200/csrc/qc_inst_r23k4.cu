@@ -40,12 +40,12 @@ static const QcEntry qc_r23k4[] = {
 };
 LDPC_QC_REGISTER(qc_r23k4)
 
-// Default shapes (us of the kernel at 1 / 100 / 440 / 25000 frames, 2.85 dB):
-//   bf16: layout 6 36.2 / 43.3 / 84.3 / 3731, layout 2 40.1 / 46.6 / 110.6 / 5068, (1,1,0,0) 37.2 / 45.4 / 114.0 / 5451;
-//         min-sum (10000 frames) 28.8 / 37.0 / 74.0 / 1312 against 31.1 / 41.1 / 94.6 / 1800; with clips 39.2 / 45.2 / 92.5 / 1676
-//         against 41.2 / 47.3 / 121.2 / 2347
-//   fp16: layout 6 39.1 / 45.4 / 90.5 / 3737, layout 2 38.9 / 45.4 / 107.8 / 4951, (1,1,0,0) 37.2 / 43.2 / 110.9 / 5189
-//   fp32: layout 6 34.9 / 41.2 / 78.2 / 3366, layout 2 36.1 / 43.3 / 99.4 / 4509, (1,1,0,0) 33.2 / 39.8 / 99.6 / 4664
+// Default shapes.  us of the kernel at 1 / 100 / 440 / 1500 / 25000 frames, 2.85 dB, all shapes in one run:
+//   bf16: layout 6 30.7 / 40.7 / 81.9 / 238 / 3529, layout 2 34.4 / 43.0 / 86.0 / 249 / 3543, (1,1,0,0) 32.8 / 43.0 / 114 / 354 / 5454;
+//         min-sum 28.7 / 34.8 / 73.7 / 223 / 3242 and (1,1,0,0) 30.7 / 38.9 / 97.3 / 296 / 4474; with clips 33.7 / 43.8 / 90.1 / 281 / 4151
+//         and 35.8 / 46.3 / 121 / 377 / 5860
+//   fp16: layout 6 34.8 / 43.0 / 90.1 / 272 / 3741, layout 2 34.8 / 43.0 / 107 / 328 / 4958, (1,1,0,0) 32.8 / 43.0 / 109 / 338 / 5198
+//   fp32: layout 6 28.7 / 37.6 / 74.8 / 216 / 3167, layout 2 30.7 / 38.9 / 95.2 / 286 / 4293, (1,1,0,0) 29.7 / 38.9 / 98.3 / 305 / 4669
 static const QcDefault qc_r23k4_default[] = {
     {256, 10, STORE_BF16, -1, 0, 1, 1, 2, 6},
     {256, 10, STORE_BF16, -1, 200, 1, 1, 0, 2},

@@ -60,21 +60,23 @@ static const QcEntry qc_r45k1[] = {
     // clips with fp16 and fp32 storage, caller-supplied LLRs (also the decoding without allocation)
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP16, ALGO_AMIN, true, true, 16),
     LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, true, true, 24),
-    // fp32 caller-supplied LLRs at LLR_SCALE (the unscaled counterpart is the larger cap): us for 8000 / 300 frames with 16
-    // CTAs' registers 293 / 65.5, 18 310 / 67.6, 20 310 / 65.5, 22 329 / 69
-    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 16),
+    // fp32 caller-supplied LLRs at LLR_SCALE (the unscaled counterpart is the larger cap): us for 300 / 8000 frames with 15 CTAs'
+    // registers 66.5 / 295, 16 66.5 / 293, 17 68.6 / 299, 22 69 / 329; 15, which no simulation kernel has, leaves
+    // simulations their own default
+    LDPC_QC_ENTRY_GR(32, 18, 1, 1, STORE_FP32, ALGO_AMIN, false, true, 15),
 };
 LDPC_QC_REGISTER(qc_r45k1)
 
-// Default shapes (us of the kernel at 1 / 440 / 5000 / 100000 frames, 3.80 dB): layout 7 at 16 or 24 CTAs per SM
-//   bf16: 45.2 / 84.2 / 190.8 / 3067, (1,1,0,0) 45.9 / 97.2 / 478.5 / 11184; min-sum 34.0 / 54.3 / 175.5 / 2607 against 38.3 /
-//         68.9 / 362.8 / 7348; with clips 46.4 / 87.3 / 209.8 / 4138 against 50.5 / 108.8 / 522.4 / 13509
-//   fp16: 41.9 / 78.2 / 186.3 / 3140, (1,1,0,0) 44.2 / 98.6 / 457.6 / 11299
-//   fp32: 43.2 / 80.1 / 188.7 / 2631, layout 1 43.4 / 92.2 / 289.0 / 5677
+// Default shapes.  us of the kernel at 1 / 440 / 1500 / 5000 / 100000 frames, 3.80 dB, all shapes in one run: layout 7 at 16 or 24
+// CTAs per SM
+//   bf16: 28.7 / 73.8 / 94.2 / 248 / 3423, (1,1,0,0) 33.8 / 91.0 / 143 / 534 / 11715; min-sum 27.5 / 65.5 / 143 / 870 / 2786 and 33.6 / 84.9 /
+//         187 / 1203 / 7767; with clips 30.7 / 83.9 / 1689 / 1737 / 4811 and 36.9 / 98.3 / 1939 / 2221 / 14962
+//   fp16: 28.7 / 69.4 / 124 / 358 / 3419, (1,1,0,0) 32.8 / 78.7 / 160 / 638 / 11425
+//   fp32: 24 CTAs 27.5 / 69.7 / 119 / 242 / 2405, 16 CTAs 26.7 / 65.5 / 119 / 246 / 2447, layout 1 32.4 / 77.8 / 150 / 389 / 5398
 static const QcDefault qc_r45k1_default[] = {
     {32, 18, STORE_BF16, -1, 0, 1, 1, 16, 7},
     {32, 18, STORE_FP16, -1, 0, 1, 1, 16, 7},
-    {32, 18, STORE_FP32, -1, 0, 1, 1, 16, 7},  // (caller-supplied LLRs only)
+    {32, 18, STORE_FP32, -1, 0, 1, 1, 15, 7},  // (caller-supplied LLRs only)
     {32, 18, STORE_FP32, -1, 0, 1, 1, 24, 7},
 };
 LDPC_QC_DEFAULTS(qc_r45k1_default)

@@ -88,14 +88,13 @@ static const QcEntry qc_r45k4[] = {
 };
 LDPC_QC_REGISTER(qc_r45k4)
 
-// Default shapes (us of the kernel at 1 / 100 / 440 / 25000 frames, 3.80 dB): layout 7 at 6 CTAs per SM
-//   bf16: 43.3 / 52.5 / 81.3 / 2853, (1,1,0,0) 39.0 / 51.6 / 97.5 / 5365; min-sum (10000 frames) 33.0 / 41.2 / 72.0 / 1012 against
-//         37.2 / 49.2 / 88.4 / 1567; with clips 47.4 / 55.6 / 90.8 / 1362 against 45.2 / 57.7 / 106.7 / 2404
-//   fp16: 43.2 / 49.8 / 80.0 / 2760, (1,1,0,0) 37.1 / 54.6 / 97.6 / 5218;  fp32: 42.3 / 50.5 / 84.3 / 2681, layout 1 42.3 / 53.6 /
-//         90.4 / 3705
-//   weighted, per edge (10000 frames): bf16 70.2 / 82.3 / 98.4 / 1247, (1,1,0,0) 59.6 / 70.0 / 121.4 / 2429; fp16 61.8 / 70.1 /
-//         94.7 / 1319 against 55.6 / 63.8 / 117.1 / 2372; fp32 (1500 frames: 254) 71.7 / 82.3 / 102.7 / 1418, layout 1 cap 8 (302)
-//         67.8 / 78.2 / 98.6 / 1887
+// Default shapes.  us of the kernel at 1 / 100 / 440 / 1500 / 25000 frames, 3.80 dB, all shapes in one run: layout 7 at 6 CTAs per SM
+//   bf16: 35.8 / 50.0 / 75.7 / 199 / 2729, (1,1,0,0) 38.8 / 53.2 / 96.3 / 303 / 5349; min-sum 32.7 / 38.8 / 69.6 / 181 / 2471 and 37.9 / 46.0 /
+//         86.0 / 246 / 3913; with clips 40.9 / 55.3 / 88.1 / 242 / 4054 and 41.0 / 55.3 / 104 / 339 / 6325
+//   fp16: 36.9 / 51.0 / 78.8 / 202 / 2767, (1,1,0,0) 37.7 / 52.0 / 93.1 / 296 / 5175;  fp32: 34.8 / 47.9 / 78.6 / 197 / 2600, layout 1 38.9 /
+//         53.2 / 86.0 / 254 / 3677
+//   weighted, per edge: bf16 72.4 / 84.8 / 99.1 / 225 / 3012, (1,1,0,0) 63.5 / 73.8 / 115 / 343 / 6103; fp16 62.2 / 72.4 / 93.0 / 236 / 3210 and
+//         59.4 / 68.4 / 111 / 338 / 5963; fp32 72.5 / 84.0 / 103 / 256 / 3458, layout 1 cap 8 69.6 / 81.9 / 102 / 303 / 4706
 static const QcDefault qc_r45k4_default[] = {
     {128, 18, STORE_FP32, ALGO_WAMIN, 1000, 1, 1, 6, 7},
     {128, 18, STORE_FP32, ALGO_WAMIN, 0, 1, 1, 8, 1},
