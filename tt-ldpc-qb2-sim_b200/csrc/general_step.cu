@@ -142,11 +142,9 @@ __global__ void __launch_bounds__(32, STEP_MIN_CTAS) general_step_kernel(const _
             float ch_mu = p.mu, ch_sigma = p.sigma;
             if (per_frame_snr)
                 frame_snr(p.ebn0_lo, p.ebn0_hi, p.rate, gf, p.stream, p.seed_lo, p.seed_hi, ch_mu, ch_sigma, snr_bin);
-            float l_max = p.l_max;
             if (SC) {
                 ch_mu *= LLR_SCALE;
                 ch_sigma *= LLR_SCALE;
-                l_max *= LLR_SCALE;
             }
             for (int qd = lane; qd * 4 < p.n_tx; qd += 32) {
                 float nz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -160,7 +158,10 @@ __global__ void __launch_bounds__(32, STEP_MIN_CTAS) general_step_kernel(const _
                 for (int k = 0; k < 4; ++k) {
                     if (4 * qd + k >= p.n_tx) break;
                     float x = ch_sigma > 0.0f ? __fmaf_rn(ch_sigma, nz[k], ch_mu) : ch_mu;
-                    if (l_max > 0.0f) x = fminf(fmaxf(x, -l_max), l_max);
+                    if (p.l_max > 0.0f) {
+                        const float l_max = SC ? p.l_max * LLR_SCALE : p.l_max;
+                        x = fminf(fmaxf(x, -l_max), l_max);
+                    }
                     LT::st(L, __ldg(slot + 4 * qd + k), x);
                 }
             }
