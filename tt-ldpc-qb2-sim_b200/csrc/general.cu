@@ -499,7 +499,7 @@ int launch_general(GeneralCode* g, const ldpc_run_params* p, bool ext, uint32_t 
 //
 // A matrix with the quasi-cyclic structure runs on the QC kernel (run_static_qc): its messages stay in
 // registers or take one slot per CTA, it needs no row schedule, and a frame has a whole CTA instead of one
-// warp.  LLRs in range run on the scaled kernels; all else on the variants with the clips compiled in, whatever
+// warp.  Frames with LLRs in range run on the scaled kernels; all else on the variants with the clips compiled in, whatever
 // the clips (with infinite caps they change only a NaN posterior, to -inf, as the general kernel does).  4001
 // frames r1/2 K=1024 bf16 2.0 dB with posteriors: 3.00 ms on the general kernel (1.41 of them the schedule of
 // that time), 0.27.
